@@ -17,8 +17,9 @@
 //   k_cavity    one warp per surviving nominee: search of the conflict region
 //               from the simplex that contains it (`locate` +
 //               `find_all_neighbors`, src/delaunay_tree.rs:33-75) with exact
-//               perturbed in-sphere tests, collection of the boundary facets
-//               (`get_new_simplices`, :77-123), then atomicMin claims with the
+//               perturbed in-sphere tests (3D: the stored circumsphere first,
+//               the vertices where it cannot decide), the boundary facets
+//               (`get_new_simplices`, :77-123) as they are met, then atomicMin claims with the
 //               candidate's priority on the cavity (claim_c) and, in the
 //               strict round mode, on every outer neighbour (claim_n).
 //               Regions that outgrow a warp's shared memory are searched
@@ -32,7 +33,8 @@
 //               mode a decide half and a commit half are separate kernels, and
 //               the stars of winners that share a facet are stitched at the
 //               start of k_relocate.  A round equals some sequential insertion
-//               order.
+//               order.  k_reclaim (and k_relocate for the last pass) also makes
+//               the stored spheres of the stars just written.
 //   k_relocate  one thread per uninserted point: points whose simplex was
 //               removed walk inside the new star (faces through the new vertex
 //               only) to the simplex that contains them; every point then votes
@@ -129,6 +131,77 @@ __device__ __forceinline__ vdp::FPt load_fpt(const DevTree& T, int v) {
   return vdp::FPt{h.x, h.y, h.z, h.w, l.x, l.y, l.z, l.w};
 }
 
+// First tier of the test of point q (record fq) against simplex nb, whose record
+// is returned in vv, nn: +1 in conflict, -1 not, 0 undecided.  The stored
+// sphere is read together with the record: one round trip and 48 bytes, where
+// the vertices' split coordinates take a second, dependent round trip and 128
+// bytes more.
+template <int D>
+__device__ __forceinline__ int sphere_tier(const DevTree& T, int nb, int4& vv, int4& nn, const vdp::FPt& fq) {
+  const float4 sp = *reinterpret_cast<const float4*>(T.sph + nb);  // nb is in range: the callers check
+  load_simplex(T, nb, vv, nn);
+  return vdp::sphere_side<D>(vdp::Sph{sp.x, sp.y, sp.z, sp.w}, fq);
+}
+// The tiers of a conflict test behind the stored sphere (split coordinates,
+// FP64, exact): simplex vertices vv, point qv (record fq).
+template <int D, int XT>
+__device__ __forceinline__ bool conflict_tiers(const DevTree& T, int4 vv, const vdp::FPt& fq, int qv, vdp::Tally& tl,
+                                               int& perr) {
+  constexpr int NV = D + 1;
+  vdp::FPt fv[NV];
+  int kv[NV];
+  for (int j = 0; j < NV; ++j) {
+    kv[j] = get4(vv, j);
+    fv[j] = load_fpt(T, kv[j]);
+  }
+  auto load64 = [&](vdp::VPt* v64, vdp::VPt& q64) {
+    for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, kv[j]);
+    q64 = load_pt(T, qv);  // reloaded: the rare FP64 path need not hold q in registers
+  };
+  return vdp::in_conflict_hl<D, XT>(fv, kv, fq, qv, tl, perr, load64);
+}
+
+// Boundary facet records (6 ints, 8-byte aligned): the vertices of the new
+// simplex on the facet, the code of the simplex outside it, and
+// (k << 4) | (qf << 2) | f: face f of cavity simplex k, the new point at
+// position qf of the new simplex.
+__device__ __forceinline__ int rec_k(int r5) { return r5 >> 4; }
+__device__ __forceinline__ int rec_q(int r5) { return (r5 >> 2) & 3; }
+__device__ __forceinline__ int rec_f(int r5) { return r5 & 3; }
+__device__ __forceinline__ void put_facet(int* F, int j, int4 nv, int code, int r5) {
+  int2* r = reinterpret_cast<int2*>(F + 6 * j);
+  r[0] = make_int2(nv.x, nv.y);
+  r[1] = make_int2(nv.z, nv.w);
+  r[2] = make_int2(code, r5);
+}
+// The record of face f of cavity simplex k whose outer simplex (code, vertices
+// vv) is not in conflict: that simplex with the vertex behind the facet
+// replaced by the new point has the wrong orientation (the point lies on the
+// other side), so two of the facet's vertices change places.
+template <int D>
+__device__ __forceinline__ int4 facet_simplex(int4 vv, int g, int qv) {
+  int4 a = set4(vv, g, qv);
+  if (D == 3) {
+    const bool mid = g == 0 || g == 3;  // swap positions g ^ 1 and g ^ 2
+    return mid ? make_int4(a.x, a.z, a.y, a.w) : make_int4(a.w, a.y, a.z, a.x);
+  }
+  return g == 0 ? make_int4(a.x, a.z, a.y, a.w) : (g == 1 ? make_int4(a.z, a.y, a.x, a.w) : make_int4(a.y, a.x, a.z, a.w));
+}
+
+// Stored sphere of the simplex with vertices r[0..D], one of which (position
+// qf) is the new point, whose record is fq: the base of the differences.
+template <int D>
+__device__ __forceinline__ void store_sphere(const DevTree& T, int s, const int* r, int qf, const vdp::FPt& fq) {
+  constexpr int NV = D + 1;
+  vdp::FPt v[NV];
+  v[0] = fq;
+#pragma unroll
+  for (int i = 0; i < D; ++i) v[i + 1] = load_fpt(T, r[i + (i >= qf ? 1 : 0)]);  // the D positions other than qf
+  if (bad_simp(T, s)) return;
+  const vdp::Sph c = vdp::sphere_of<D>(v);
+  *reinterpret_cast<float4*>(T.sph + s) = make_float4(c.x, c.y, c.z, c.w);
+}
+
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
   for (int o = 16; o; o >>= 1) v += __shfl_down_sync(FULL, v, o);
   return v;
@@ -139,7 +212,8 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 // 1M-point build).  Counts that steer the build (winners, inserted) are
 // summed per block instead (shared memory, one atomic per block).
 __device__ void flush_tally(Counters* c, const vdp::Tally& t, unsigned tests, unsigned walk) {
-  const unsigned long long v[STAT_COUNT] = {warp_sum(t.f32), warp_sum(t.f64), warp_sum(t.exact),
+  // f32 as a signed number: a lane's share of it may be below zero (SearchStats::merge)
+  const unsigned long long v[STAT_COUNT] = {warp_sum((unsigned long long)(long long)(int)t.f32), warp_sum(t.f64), warp_sum(t.exact),
                                             warp_sum(t.sos), warp_sum(tests), warp_sum(walk)};
   if ((threadIdx.x & 31) == 0) {
     const unsigned stripe = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) % kStatStripes;
@@ -548,23 +622,47 @@ __device__ __forceinline__ int load_heads(const DevTree& T, HeadBuf& H, const in
   return n;
 }
 
+// Decisions of a warp's searches beyond the sphere tier (which decides every
+// test that is not counted as undecided), in shared memory: they are rare, and
+// as registers they would live through every wave.
+struct SearchStats {
+  unsigned f32, f64, exact, sos, undecided;
+  int perr;
+  unsigned spilled;
+  __device__ void clear() {
+    f32 = f64 = exact = sos = undecided = spilled = 0;
+    perr = 0;
+  }
+  // Into lane 0's tally at the end; ntests are the lane's own tests.
+  template <int D>
+  __device__ void merge(vdp::Tally& t, int& p, unsigned ntests, int lane) const {
+    if (D == 3) t.f32 += ntests;
+    if (lane) return;
+    t.f32 += f32 - undecided;
+    t.f64 += f64;
+    t.exact += exact;
+    t.sos += sos;
+    p |= perr;
+  }
+};
+
 // Storage of one cavity search: shared memory for the common case, a
 // reserved, 16-byte aligned stretch of the round's cavity pool when that
 // overflows.  Generic pointers let the same code run on both.
 struct CavStore {
   int* cav;     // simplex ids of the conflict region
-  int4* cv;     // their vertex ids
   int4* cn;     // their neighbour codes
-  int* hk;      // open-addressing set of cavity ids (hs slots, power of two)
-  int2* fr;     // boundary facets: (outer code, (k << 2) | face); expanded to
-                // 6-int records (new simplex vertices, outer code, (k << 2) | face)
-                // when the lists are stored
+  int* hk;      // open-addressing set of cavity ids (hs slots, power of two, a multiple of 128)
+  int* F;       // boundary facet records (put_facet), in the pool
+  int* und;     // items that the sphere tier left undecided (kUndecided)
+  SearchStats* st;
   int maxc, maxf, hs;
 };
 
-// Spill stretch layout (ints): cavity ids | facet records | cv | cn | id set |
-// ridge table (keys 2 ints + partners 2 ints per slot).  The search uses the
-// first five parts, the commit of a large star the facets and the ridge table.
+// Spill stretch layout (ints): cavity ids | facet records | new ids | cn | id
+// set | ridge table (keys 2 ints + partners 2 ints per slot).  The search uses
+// the ids, facets, cn and id set, the commit of a large star the facets, the new
+// ids and the ridge table.
 constexpr int kBigC = 8192, kBigF = 12288, kBigH = 32768, kBigR = 65536;
 // Fresh simplex slots a warp takes at a time in k_check.
 constexpr int kSlotChunk = 32;
@@ -577,9 +675,9 @@ constexpr int kBigInts = kOffR + 4 * kBigR;  // multiple of 4
 // Dynamic shared memory of k_cavity_big: the id set (kBigH ints) and the
 // ready marks (kBigC ints) of its block search.
 constexpr int kBigSmem = (kBigH + kBigC) * (int)sizeof(int);
-// Offset of the facet records after ncav cavity ids: even, so that records
-// (6 ints) start on 8-byte boundaries in an even pool stretch.
-__host__ __device__ constexpr int facets_at(int ncav) { return (ncav + 1) & ~1; }
+// Pool ints of a searched region: its facet records (6 ints each), then its
+// cavity ids, rounded up to even so that records stay on 8-byte boundaries.
+__host__ __device__ constexpr int region_ints(int ncav, int nfac) { return (6 * nfac + ncav + 1) & ~1; }
 
 __device__ bool hset_insert(int* hk, int hs, int key) {
   unsigned h = ((unsigned)key * 2654435761u) & (hs - 1);
@@ -602,6 +700,25 @@ __device__ bool hset_find(const int* hk, int hs, int key) {
   return false;
 }
 
+// Facet record s of item (k, f) of a search: `sk` is cavity simplex k, code the
+// simplex outside (vertices vv), or negative on the super-simplex hull, where
+// the new simplex is simplex k with its vertex f replaced.
+template <int D>
+__device__ __forceinline__ void put_item_facet(const DevTree& T, int* F, int s, int4 vv, int code, int sk, int k, int f,
+                                               int qv) {
+  if (code < 0) {
+    int4 kv, kn;
+    load_simplex(T, sk, kv, kn);
+    put_facet(F, s, set4(kv, f, qv), code, (k << 4) | (f << 2) | f);
+  } else {
+    const int g = code & 3;
+    put_facet(F, s, facet_simplex<D>(vv, g, qv), code, (k << 4) | (g << 2) | f);
+  }
+}
+
+// Undecided items a warp collects before it settles them.
+constexpr int kUndecided = 64;
+
 struct WarpCtl {
   int ncav, nfac, flags, pad;
   int head, pend;  // block search: next item to hand out, items created and not finished
@@ -622,8 +739,8 @@ constexpr long long kDynWaitLimit = 1LL << 24;
 // and capacity flags as the wave form; only the order of the lists differs.
 template <int D, int XT>
 __device__ void cavity_search_dyn(const DevTree& T, const CavStore& S, WarpCtl& ctl, int* rdy, int rank,
-                                  int start, int4 v0, int4 n0, int qv, const vdp::FPt& fq, vdp::Tally& tl,
-                                  int& perr, unsigned& ntests) {
+                                  int start, int4 n0, int qv, const vdp::FPt& fq, vdp::Tally& tl, int& perr,
+                                  unsigned& ntests) {
   constexpr int NV = D + 1;
   const int G = (int)blockDim.x;
   for (int i = rank; i < S.hs; i += G) S.hk[i] = -1;
@@ -636,7 +753,6 @@ __device__ void cavity_search_dyn(const DevTree& T, const CavStore& S, WarpCtl& 
     ctl.head = 0;
     ctl.pend = NV;
     S.cav[0] = start;
-    S.cv[0] = v0;
     S.cn[0] = n0;
     hset_insert(S.hk, S.hs, start);
     rdy[0] = 1;
@@ -664,30 +780,25 @@ __device__ void cavity_search_dyn(const DevTree& T, const CavStore& S, WarpCtl& 
     __threadfence_block();  // the entry's records after its ready mark
     const int code = get4(__ldcg(&S.cn[k]), f);  // from L2: another thread stored it
     bool facet = code < 0;
+    int4 vv = make_int4(-1, -1, -1, -1), nn;
     const bool broken = !facet && bad_simp(T, code >> 2);
     if (broken) set_error(T.ctr, E_INTERNAL);
     if (!facet && !broken) {
       const int nb = code >> 2;
       if (!hset_find(S.hk, S.hs, nb)) {
-        int4 vv, nn;
-        load_simplex(T, nb, vv, nn);
-        vdp::FPt fv[NV];
-        int kv[NV];
-        for (int j = 0; j < NV; ++j) {
-          kv[j] = get4(vv, j);
-          fv[j] = load_fpt(T, kv[j]);
-        }
         ++ntests;
-        auto load64 = [&](vdp::VPt* v64, vdp::VPt& q64) {
-          for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, kv[j]);
-          q64 = load_pt(T, qv);
-        };
-        if (vdp::in_conflict_hl<D, XT>(fv, kv, fq, qv, tl, perr, load64)) {
+        int side = 0;
+        if (D == 3) {
+          side = sphere_tier<D>(T, nb, vv, nn, fq);
+          tl.f32 += side != 0;
+        } else {
+          load_simplex(T, nb, vv, nn);
+        }
+        if (side > 0 || (side == 0 && conflict_tiers<D, XT>(T, vv, fq, qv, tl, perr))) {
           if (hset_insert(S.hk, S.hs, nb)) {
             const int s = atomicAdd(&ctl.ncav, 1);
             if (s < S.maxc) {
               S.cav[s] = nb;
-              S.cv[s] = vv;
               S.cn[s] = nn;
               atomicAdd(&ctl.pend, NV);  // before the mark: the parent item is still counted
               __threadfence_block();
@@ -703,7 +814,7 @@ __device__ void cavity_search_dyn(const DevTree& T, const CavStore& S, WarpCtl& 
     }
     if (facet) {
       const int s = atomicAdd(&ctl.nfac, 1);
-      if (s < S.maxf) S.fr[s] = make_int2(code, (k << 2) | f);
+      if (s < S.maxf) put_item_facet<D>(T, S.F, s, vv, code, __ldcg(&S.cav[k]), k, f, qv);
       else atomicOr(&ctl.flags, 2);
     }
     atomicSub(&ctl.pend, 1);
@@ -711,110 +822,158 @@ __device__ void cavity_search_dyn(const DevTree& T, const CavStore& S, WarpCtl& 
   __syncthreads();
 }
 
-// Breadth-first search of the conflict region of candidate q from the
-// simplex that contains it; all 32 lanes of the warp call this.  Returns
-// with ctl.flags != 0 if a capacity was exceeded.
+// Search of the conflict region of candidate q from the simplex that contains
+// it by one warp; returns the region's size, its boundary facets and whether a
+// capacity was exceeded (the same in every lane).
 //
-// BLOCK: the whole block searches (k_cavity_big, lane = thread index, waves
-// of blockDim.x items); ctl.pad carries the wave's item count, published by
-// thread 0 so that every thread leaves the loop after the same barrier.
-template <int D, int XT, bool BLOCK = false>
-__device__ void cavity_search(const DevTree& T, const CavStore& S, WarpCtl& ctl, int lane, int start,
-                              int4 v0, int4 n0, int qv, const vdp::FPt& fq, vdp::Tally& tl, int& perr,
-                              unsigned& ntests) {
+// (simplex, face) items are taken in waves of 32 in discovery order, not level
+// by level: a wave also takes the items of simplices the previous wave
+// appended, so a search needs about items / 32 dependent round trips rather
+// than one or more per level.  A wave's appends are counted by ballots: one
+// shared-memory atomic per new simplex (its entry in the id set) and none on
+// the list lengths.
+//
+// What bounds it: a wave's one round trip (about 1,000 cycles) and about 200
+// instructions, on 20 warps per SM; 24 and 32 warps per SM at fewer registers
+// were slower (spills), 16 without spills too (tail).  The 1M-point build's
+// searches took 13.2 ms with vertex tests in the wave, 10.2 ms in this form;
+// near-degenerate 262,144 points 21.1 and 15.4 ms (CUDA events per kernel).
+//
+// In 3D the waves hold the sphere tier alone.  Items that it cannot decide are
+// set aside and settled in batches by the other tiers (settle_items), out of
+// the loop: their code is large, and inside the loop it set the registers of
+// every wave.  In 2D the other tiers stay in the wave and there are no stored
+// spheres: a circle saves three vertex records of a test and costs as much to
+// make for each new triangle (1M points: 17.4 ms with, 16.3 without).
+struct Region {
+  int ncav, nfac;
+  bool over;
+};
+
+// Appends of one wave: lanes with `add` put simplex nb into the region, lanes
+// with `facet` write the record of item (k, f).  False when a list is full.
+template <int D>
+__device__ __forceinline__ bool append_wave(const DevTree& T, const CavStore& S, Region& R, unsigned below, bool add,
+                                            bool facet, int nb, int4 vv, int4 nn, int code, int k, int f, int qv) {
+  const unsigned ma = __ballot_sync(FULL, add), mf = __ballot_sync(FULL, facet);
+  const int na = R.ncav + __popc(ma), nf = R.nfac + __popc(mf);
+  if (na > S.maxc || nf > S.maxf) {
+    R.ncav = na;
+    R.nfac = nf;
+    R.over = true;
+    return false;
+  }
+  if (add) {
+    const int s = R.ncav + __popc(ma & below);
+    S.cav[s] = nb;
+    S.cn[s] = nn;
+  }
+  if (facet) put_item_facet<D>(T, S.F, R.nfac + __popc(mf & below), vv, code, S.cav[k], k, f, qv);
+  __syncwarp();
+  R.ncav = na;
+  R.nfac = nf;
+  return true;
+}
+
+// Settles the nu undecided items of a search; appends to the region.
+template <int D, int XT>
+__device__ __forceinline__ void settle_items(const DevTree& T, const CavStore& S, Region& R, int lane, int nu, int qv,
+                                             const vdp::FPt& fq) {
   constexpr int NV = D + 1;
-  const int G = BLOCK ? (int)blockDim.x : 32;
-  auto sync = [] {
-    if (BLOCK)
-      __syncthreads();
-    else
-      __syncwarp();
-  };
-  for (int i = lane; i < S.hs; i += G) S.hk[i] = -1;
+  const unsigned below = (1u << lane) - 1;
+  vdp::Tally tl = {0, 0, 0, 0};
+  int perr = 0;
+  for (int i0 = 0; i0 < nu; i0 += 32) {
+    const bool act = i0 + lane < nu;
+    const int it = act ? S.und[i0 + lane] : 0;
+    const int k = it / NV, f = it - k * NV;
+    const int code = reinterpret_cast<const int*>(S.cn + k)[f];
+    const int nb = code >> 2;
+    bool add = false, facet = false;
+    int4 vv = make_int4(-1, -1, -1, -1), nn = vv;
+    if (act && !hset_find(S.hk, S.hs, nb)) {
+      load_simplex(T, nb, vv, nn);
+      if (conflict_tiers<D, XT>(T, vv, fq, qv, tl, perr))
+        add = hset_insert(S.hk, S.hs, nb);
+      else
+        facet = true;
+    }
+    __syncwarp();
+    if (!append_wave<D>(T, S, R, below, add, facet, nb, vv, nn, code, k, f, qv)) break;
+  }
+  SearchStats& st = *S.st;
+  if (lane == 0) atomicAdd(&st.undecided, (unsigned)nu);
+  if (tl.f32) atomicAdd(&st.f32, tl.f32);
+  if (tl.f64) atomicAdd(&st.f64, tl.f64);
+  if (tl.exact) atomicAdd(&st.exact, tl.exact);
+  if (tl.sos) atomicAdd(&st.sos, tl.sos);
+  if (perr) atomicOr(&st.perr, perr);
+}
+
+template <int D, int XT>
+__device__ __forceinline__ Region cavity_search(const DevTree& T, const CavStore& S, int lane, int start, int4 n0,
+                                                int qv, const vdp::FPt& fq, vdp::Tally& tl, int& perr,
+                                                unsigned& ntests) {
+  constexpr int NV = D + 1;
+  for (int i = lane; i < S.hs / 4; i += 32) reinterpret_cast<int4*>(S.hk)[i] = make_int4(-1, -1, -1, -1);
+  __syncwarp();
   if (lane == 0) {
-    ctl.ncav = 1;
-    ctl.nfac = 0;
-    ctl.flags = 0;
     S.cav[0] = start;
-    S.cv[0] = v0;
     S.cn[0] = n0;
+    hset_insert(S.hk, S.hs, start);
   }
-  sync();
-  if (lane == 0) hset_insert(S.hk, S.hs, start);
-  sync();
-  // (simplex, face) items are taken in waves of G in discovery order, not
-  // level by level: a wave also takes the items of simplices the previous
-  // wave appended, so a search needs about items / G dependent rounds of
-  // gathers rather than one or more per level
-  int head = 0, levels = 0;
+  __syncwarp();
+  Region R{1, 0, false};
+  int head = 0, waves = 0, nu = 0;
+  const unsigned below = (1u << lane) - 1;
   while (true) {
-    int avail;
-    if (BLOCK) {
-      if (lane == 0) {
-        const int a = min(*(volatile int*)&ctl.ncav, S.maxc) * NV;
-        ctl.pad = (*(volatile int*)&ctl.flags || head >= a) ? -1 : a;
-      }
-      sync();
-      avail = *(volatile int*)&ctl.pad;
-      if (avail < 0) break;
-    } else {
-      avail = min(*(volatile int*)&ctl.ncav, S.maxc) * NV;
-      if (*(volatile int*)&ctl.flags || head >= avail) break;
-    }
-    ++levels;
-    const int it = head + lane;
-    if (it < avail) {
+    while (head < R.ncav * NV && nu <= kUndecided - 32) {
+      ++waves;
+      const int it = head + lane;
+      const int avail = R.ncav * NV;
+      const bool act = it < avail;
       const int k = it / NV, f = it - k * NV;
-      const int code = get4(S.cn[k], f);
-      bool facet = code < 0;
-      const bool broken = !facet && bad_simp(T, code >> 2);
-      if (broken) set_error(T.ctr, E_INTERNAL);
-      if (!facet && !broken) {
-        const int nb = code >> 2;
-        if (!hset_find(S.hk, S.hs, nb)) {
-          int4 vv, nn;
-          load_simplex(T, nb, vv, nn);
-          vdp::FPt fv[NV];
-          int kv[NV];
-          for (int j = 0; j < NV; ++j) {
-            kv[j] = get4(vv, j);
-            fv[j] = load_fpt(T, kv[j]);
-          }
-          ++ntests;
-          auto load64 = [&](vdp::VPt* v64, vdp::VPt& q64) {
-            for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, kv[j]);
-            q64 = load_pt(T, qv);  // reloaded: the rare FP64 path need not hold q in registers
-          };
-          if (vdp::in_conflict_hl<D, XT>(fv, kv, fq, qv, tl, perr, load64)) {
-            if (hset_insert(S.hk, S.hs, nb)) {
-              int s = atomicAdd(&ctl.ncav, 1);
-              if (s < S.maxc) {
-                S.cav[s] = nb;
-                S.cv[s] = vv;
-                S.cn[s] = nn;
-              } else {
-                atomicOr(&ctl.flags, 1);
-              }
-            }
-          } else {
-            facet = true;
-          }
-        }
+      int code = -1;
+      if (act) code = reinterpret_cast<const int*>(S.cn + k)[f];
+      const int nb = code >> 2;
+      bool test = code >= 0;
+      if (test && bad_simp(T, nb)) {
+        set_error(T.ctr, E_INTERNAL);
+        test = false;
       }
-      if (facet) {
-        int s = atomicAdd(&ctl.nfac, 1);
-        if (s < S.maxf) {
-          S.fr[s] = make_int2(code, (k << 2) | f);
+      bool facet = act && code < 0;
+      bool add = false, und = false;
+      int4 vv = make_int4(-1, -1, -1, -1), nn = vv;
+      if (test && !hset_find(S.hk, S.hs, nb)) {
+        ++ntests;
+        int side;
+        if constexpr (D == 3) {
+          side = sphere_tier<D>(T, nb, vv, nn, fq);
         } else {
-          atomicOr(&ctl.flags, 2);
+          load_simplex(T, nb, vv, nn);
+          side = conflict_tiers<D, XT>(T, vv, fq, qv, tl, perr) ? 1 : -1;
         }
+        und = side == 0;
+        facet = side < 0;
+        if (side > 0) add = hset_insert(S.hk, S.hs, nb);
       }
+      __syncwarp();
+      if constexpr (D == 3) {
+        const unsigned mu = __ballot_sync(FULL, und);
+        if (und) S.und[nu + __popc(mu & below)] = it;
+        nu += __popc(mu);
+      }
+      if (!append_wave<D>(T, S, R, below, add, facet, nb, vv, nn, code, k, f, qv)) break;
+      head = min(head + 32, avail);
     }
-    sync();
-    head += min(G, avail - head);
+    if (R.over || nu == 0) break;
+    settle_items<D, XT>(T, S, R, lane, nu, qv, fq);
+    nu = 0;
+    if (R.over) break;
   }
-  sync();
-  if (lane == 0 && levels > 64) atomicMax(&T.ctr->max_levels, levels);
+  if (nu && lane == 0) atomicAdd(&S.st->undecided, (unsigned)nu);
+  if (lane == 0 && waves > 64) atomicMax(&T.ctr->max_levels, waves);
+  return R;
 }
 
 // Thinning test of one nominee (one thread): it must hold the thinning claim
@@ -911,32 +1070,18 @@ template <int D>
 __global__ void k_thin(DevTree T, int thin) { thin_body<D>(T, thin, blockIdx.x, gridDim.x); }
 
 template <int D>
-struct WarpCav {
+struct alignas(16) WarpCav {
   WarpCtl ctl;
+  SearchStats st;
   int cav[Cap<D>::MAXC];
-  int4 cv[Cap<D>::MAXC];
   int4 cn[Cap<D>::MAXC];
   int hkey[Cap<D>::HS];
-  int2 fr[Cap<D>::MAXF];
+  int und[kUndecided];
 };
 
 // Claims of a candidate for one resolution pass: its cavity in claim_c, every
 // outer neighbour in claim_n (not in adjacent mode, where cavities may touch).
 // P = cavity ids, F = facet records.
-// Facet records of a search, expanded for the later kernels: the new
-// simplex on facet (k, f) has the vertices of cavity simplex k with v[f]
-// replaced by the candidate's point qv.
-__device__ __forceinline__ void expand_facets(const int2* fr, const int4* cv, int nfac, int qv, int* F, int lane) {
-  for (int j = lane; j < nfac; j += 32) {
-    const int2 e = fr[j];
-    const int4 nv4 = set4(cv[e.y >> 2], e.y & 3, qv);
-    int2* r = reinterpret_cast<int2*>(F + 6 * j);  // records start on 8-byte boundaries
-    r[0] = make_int2(nv4.x, nv4.y);
-    r[1] = make_int2(nv4.z, nv4.w);
-    r[2] = e;
-  }
-}
-
 __device__ __forceinline__ void claim_region(const DevTree& T, const int* P, int ncav, const int* F,
                                              int nfac, unsigned long long key, int lane, int adjacent) {
   for (int i = lane; i < ncav; i += 32) atomicMin(T.claim_c + P[i], key);
@@ -952,7 +1097,7 @@ __device__ __forceinline__ void claim_region(const DevTree& T, const int* P, int
 // warp (BLOCK = false) or the whole block (k_cavity_big) runs it.  The
 // stretch offset is broadcast through ctl.pad.
 template <int D, int XT, bool BLOCK>
-__device__ void big_search(const DevTree& T, WarpCtl& ctl, int* bsm, int rank, int c, int4 cd, int4 v0, int4 n0,
+__device__ void big_search(const DevTree& T, WarpCtl& ctl, SearchStats* st, int* bsm, int rank, int c, int4 cd, int4 n0,
                            const vdp::FPt& fq, unsigned long long key, int adjacent, vdp::Tally& tl, int& perr,
                            unsigned& ntests, int& mcav, int& mfac) {
   auto sync = [] {
@@ -977,19 +1122,23 @@ __device__ void big_search(const DevTree& T, WarpCtl& ctl, int* bsm, int rank, i
     return;
   }
   int* P = T.pool + off;
-  // the search's 2-int facet records go to the ridge-table area (unused
-  // until the commit) and are expanded to P + kOffF afterwards
   // the block search keeps its id set and ready marks in shared memory (bsm)
-  const CavStore big{P, reinterpret_cast<int4*>(P + kOffCV), reinterpret_cast<int4*>(P + kOffCN),
-                     BLOCK ? bsm : P + kOffH, reinterpret_cast<int2*>(P + kOffR), kBigC, kBigF, kBigH};
-  if constexpr (BLOCK)
-    cavity_search_dyn<D, XT>(T, big, ctl, bsm + kBigH, rank, cd.y, v0, n0, cd.x, fq, tl, perr, ntests);
-  else
-    cavity_search<D, XT, false>(T, big, ctl, rank, cd.y, v0, n0, cd.x, fq, tl, perr, ntests);
-  const int ncav = min(*(volatile int*)&ctl.ncav, kBigC), nfac = min(*(volatile int*)&ctl.nfac, kBigF);
-  const int flags = *(volatile int*)&ctl.flags;
+  const CavStore big{P, reinterpret_cast<int4*>(P + kOffCN), BLOCK ? bsm : P + kOffH, P + kOffF, P + kOffR, st, kBigC, kBigF, kBigH};
+  int ncav, nfac;
+  bool over;
+  if constexpr (BLOCK) {
+    cavity_search_dyn<D, XT>(T, big, ctl, bsm + kBigH, rank, cd.y, n0, cd.x, fq, tl, perr, ntests);
+    ncav = min(*(volatile int*)&ctl.ncav, kBigC);
+    nfac = min(*(volatile int*)&ctl.nfac, kBigF);
+    over = *(volatile int*)&ctl.flags != 0;
+  } else {
+    const Region rg = cavity_search<D, XT>(T, big, rank, cd.y, n0, cd.x, fq, tl, perr, ntests);
+    ncav = min(rg.ncav, kBigC);
+    nfac = min(rg.nfac, kBigF);
+    over = rg.over;
+  }
   sync();
-  if (flags) {
+  if (over) {
     if (rank == 0) {
       T.cinfo[c] = make_int4(ncav, nfac, 0, ST_OVERFLOW);
       atomicAdd(&T.ctr->overflow, 1);
@@ -999,15 +1148,6 @@ __device__ void big_search(const DevTree& T, WarpCtl& ctl, int* bsm, int rank, i
   }
   // the facets stay at P + kOffF; cinfo.y carries the flag (see cand_lists)
   const int G = BLOCK ? (int)blockDim.x : 32;
-  for (int j = rank; j < nfac; j += G) {
-    const int2 e = big.fr[j];
-    const int4 nv4 = set4(big.cv[e.y >> 2], e.y & 3, cd.x);
-    int2* r = reinterpret_cast<int2*>(P + kOffF + 6 * j);
-    r[0] = make_int2(nv4.x, nv4.y);
-    r[1] = make_int2(nv4.z, nv4.w);
-    r[2] = e;
-  }
-  sync();
   for (int i = rank; i < ncav; i += G) atomicMin(T.claim_c + P[i], key);
   if (!adjacent)
     for (int j = rank; j < nfac; j += G) {
@@ -1031,22 +1171,26 @@ __device__ __forceinline__ void cavity_body(DevTree T, int adjacent, int bid, in
   vdp::Tally tl = {0, 0, 0, 0};
   int perr = 0;
   unsigned ntests = 0;
-  unsigned long long nsearched = 0, nspill = 0;
   int mcav = 0, mfac = 0;
+  if (lane == 0) W.st.clear();
+  __syncwarp();
   // pool space is taken in per-warp chunks (one atomic per chunk, not per
-  // candidate); what a warp leaves unused is dropped with the round's pool
-  const int pchunk = max(256, min(8192, T.cap_pool / (nblk * 16))) & ~1;  // offsets stay even
+  // candidate), each with room for the largest region a warp holds, since the
+  // search writes its facet records there as it finds them; what a warp
+  // leaves unused is dropped with the round's pool
+  constexpr int kMost = region_ints(MAXC, MAXF);
+  const int pchunk = max(kMost, min(8192, T.cap_pool / (nblk * 16))) & ~1;  // offsets stay even
   int pbase = 0, pleft = 0;
-  const CavStore fast{W.cav, W.cv, W.cn, W.hkey, W.fr, MAXC, MAXF, HS};
   const int nw = nblk * 4;
   const int nsurv = T.ctr->nwl[0];
+  const int* list = T.wl[0];
   // the list entry and candidate record of the warp's next item are read one
   // search ahead, so that a search starts with one round trip (its point and
   // start simplex) instead of three
   int it = bid * 4 + wib;
-  int c_next = it < nsurv ? T.wl[0][it] : 0;
+  int c_next = it < nsurv ? list[it] : 0;
   int4 cd_next = it < nsurv ? T.cand[c_next] : make_int4(0, 0, 0, 0);
-  int c_after = it + nw < nsurv ? T.wl[0][it + nw] : 0;
+  int c_after = it + nw < nsurv ? list[it + nw] : 0;
   for (; it < nsurv; it += nw) {
     const int c = c_next;
     const int4 cd = cd_next;
@@ -1057,51 +1201,44 @@ __device__ __forceinline__ void cavity_body(DevTree T, int adjacent, int bid, in
       c_next = c_after;
       cd_next = T.cand[c_after];
     }
-    if (it + 2 * nw < nsurv) c_after = T.wl[0][it + 2 * nw];
-    if (lane == 0) ++nsearched;
+    if (it + 2 * nw < nsurv) c_after = list[it + 2 * nw];
     const unsigned long long key = pe | (unsigned)cd.z;
-    cavity_search<D, XT>(T, fast, W.ctl, lane, cd.y, v0, n0, cd.x, fq, tl, perr, ntests);
-    int ncav = min(W.ctl.ncav, MAXC), nfac = min(W.ctl.nfac, MAXF);
-    int off = 0;
-    if (W.ctl.flags) {
+    if (pleft < kMost) {
+      if (lane == 0) pbase = atomicAdd(&T.ctr->pool_used, pchunk);
+      pbase = __shfl_sync(FULL, pbase, 0);
+      pleft = pbase >= 0 && (long long)pbase + pchunk <= T.cap_pool ? pchunk : 0;
+    }
+    if (pleft < kMost) {
+      if (lane == 0) {
+        T.cinfo[c] = make_int4(0, 0, 0, ST_POOL);
+        atomicAdd(&T.ctr->pool_overflow, 1);
+      }
+      __syncwarp();
+      continue;
+    }
+    int* F = T.pool + pbase;
+    const CavStore fast{W.cav, W.cn, W.hkey, F, W.und, &W.st, MAXC, MAXF, HS};
+    const Region rg = cavity_search<D, XT>(T, fast, lane, cd.y, n0, cd.x, fq, tl, perr, ntests);
+    if (rg.over) {
       // spill: the region outgrew shared memory; the search is redone in a
       // reserved pool stretch, by the whole block of k_cavity_big or here
-      if (lane == 0) ++nspill;
+      if (lane == 0) W.st.spilled += 1;
       if (defer_big) {
         if (lane == 0) {
           T.bigc[atomicAdd(&T.ctr->nbig, 1)] = c;
           T.cinfo[c] = make_int4(0, 0, 0, ST_BIG);
         }
       } else {
-        big_search<D, XT, false>(T, W.ctl, nullptr, lane, c, cd, v0, n0, fq, key, adjacent, tl, perr, ntests, mcav,
+        big_search<D, XT, false>(T, W.ctl, &W.st, nullptr, lane, c, cd, n0, fq, key, adjacent, tl, perr, ntests, mcav,
                                  mfac);
       }
       __syncwarp();
       continue;
     }
-    const int need = facets_at(ncav) + nfac * 6;
-    if (need > pleft) {
-      const int take = max(need, pchunk);
-      if (lane == 0) pbase = atomicAdd(&T.ctr->pool_used, take);
-      pbase = __shfl_sync(FULL, pbase, 0);
-      pleft = take;
-      if (pbase + take > T.cap_pool) pleft = 0;
-    }
-    if (need > pleft) {
-      if (lane == 0) {
-        T.cinfo[c] = make_int4(ncav, nfac, 0, ST_POOL);
-        atomicAdd(&T.ctr->pool_overflow, 1);
-      }
-      __syncwarp();
-      continue;
-    }
-    off = pbase;
+    const int ncav = rg.ncav, nfac = rg.nfac, off = pbase, need = region_ints(ncav, nfac);
     pbase += need;
     pleft -= need;
-    int* P = T.pool + off;
-    for (int i = lane; i < ncav; i += 32) P[i] = W.cav[i];
-    int* F = P + facets_at(ncav);
-    expand_facets(W.fr, W.cv, nfac, cd.x, F, lane);
+    for (int i = lane; i < ncav; i += 32) F[6 * nfac + i] = W.cav[i];
     __syncwarp();
     claim_region(T, W.cav, ncav, F, nfac, key, lane, adjacent);
     if (lane == 0) T.cinfo[c] = make_int4(ncav, nfac, off, ST_OK);
@@ -1109,19 +1246,21 @@ __device__ __forceinline__ void cavity_body(DevTree T, int adjacent, int bid, in
     mfac = max(mfac, nfac);
     __syncwarp();
   }
+  __syncwarp();
+  W.st.merge<D>(tl, perr, ntests, lane);
   if (perr) set_error(T.ctr, E_PRECISION);
   flush_tally(T.ctr, tl, ntests, 0);
   {
     __shared__ unsigned long long cs[2];
     __shared__ int cm[2];
-    nsearched = warp_sum(nsearched);
-    nspill = warp_sum(nspill);
+    const int first = bid * 4 + wib;
+    const int nsearched = first < nsurv ? (nsurv - 1 - first) / nw + 1 : 0, nspill = W.st.spilled;
     __syncthreads();
     if (threadIdx.x == 0) cs[0] = cs[1] = 0, cm[0] = cm[1] = 0;
     __syncthreads();
     if (lane == 0) {
-      if (nsearched) atomicAdd(&cs[0], nsearched);
-      if (nspill) atomicAdd(&cs[1], nspill);
+      if (nsearched) atomicAdd(&cs[0], (unsigned long long)nsearched);
+      if (nspill) atomicAdd(&cs[1], (unsigned long long)nspill);
       if (mcav) atomicMax(&cm[0], mcav);
       if (mfac) atomicMax(&cm[1], mfac);
     }
@@ -1158,7 +1297,7 @@ __global__ void __launch_bounds__(512, 1) k_cavity_big(DevTree T, int adjacent) 
     const vdp::FPt fq = load_fpt(T, cd.x);
     int4 v0, n0;
     load_simplex(T, cd.y, v0, n0);
-    big_search<D, XT, true>(T, ctl, bsm, threadIdx.x, c, cd, v0, n0, fq, pe | (unsigned)cd.z, adjacent, tl, perr, ntests,
+    big_search<D, XT, true>(T, ctl, nullptr, bsm, threadIdx.x, c, cd, n0, fq, pe | (unsigned)cd.z, adjacent, tl, perr, ntests,
                             mcav, mfac);
   }
   if (perr) set_error(T.ctr, E_PRECISION);
@@ -1169,17 +1308,18 @@ __global__ void __launch_bounds__(512, 1) k_cavity_big(DevTree T, int adjacent) 
   }
 }
 
-// Pool layout of a searched candidate: cavity ids at P, facet records at
-// P + facets_at(ncav) (8-byte aligned), or at P + kOffF for a spilled (large)
-// search, flagged by bit 30
-// of cinfo.y.
+// Pool layout of a searched candidate: facet records at F, cavity ids at P
+// behind them; of a spilled (large) search, flagged by bit 30 of cinfo.y, the
+// ids at the stretch's start and the facets at + kOffF.
+constexpr int kSpheresDone = 1 << 29;  // of cinfo.y: the star has its stored spheres
 __device__ __forceinline__ void cand_lists(const DevTree& T, const int4& info, int*& P, int*& F, int& ncav,
                                            int& nfac, bool& big) {
-  P = T.pool + info.z;
+  int* b = T.pool + info.z;
   ncav = info.x;
   big = (info.y >> 30) & 1;
-  nfac = info.y & ((1 << 30) - 1);
-  F = big ? P + kOffF : P + facets_at(ncav);
+  nfac = info.y & (kSpheresDone - 1);
+  P = big ? b : b + 6 * nfac;
+  F = big ? b + kOffF : b;
 }
 
 template <int D>
@@ -1218,10 +1358,13 @@ __device__ __forceinline__ void ridge_of(const int* r, int g, int qf, int& r0, i
 // neighbour that another winner of this round removed (adjacent mode) is left
 // alone: the two new simplices on that facet are linked at the start of
 // k_relocate (fix_body).
-__device__ __forceinline__ bool emit_simplex(const DevTree& T, const int* r, int myid, int4 nn, int round) {
+template <int D, bool SPH>
+__device__ __forceinline__ bool emit_simplex(const DevTree& T, const int* r, int myid, int4 nn, int round,
+                                             const vdp::FPt& fq) {
   const int4 v = make_int4(r[0], r[1], r[2], r[3]);
-  const int qf = r[5] & 3, o = r[4];
+  const int qf = rec_q(r[5]), o = r[4];
   store_simplex(T, myid, v, nn);
+  if (SPH) store_sphere<D>(T, myid, r, qf, fq);
   if (o < 0 || bad_simp(T, o >> 2)) return false;
   if (T.killed[o >> 2].x == round) return true;  // another winner's cavity: linked by fix_body
   reinterpret_cast<int*>(T.simp + (o >> 2))[4 + (o & 3)] = (myid << 2) | qf;
@@ -1242,7 +1385,7 @@ __device__ __forceinline__ unsigned ridge_hash(int r0, int r1) {
 }
 // Returns, per lane, a bit for each of its facets (j = lane, lane + 32, ...)
 // whose outer neighbour another winner of this round removed.
-template <int D>
+template <int D, bool SPH>
 __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __restrict__ FR, int nfac, int qv,
                                int round, int lane) {
   constexpr int NV = D + 1;
@@ -1251,10 +1394,11 @@ __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __
   constexpr int PER_SWEEP = 2 * HR / 3;
   const unsigned long long EMPTY = ~0ull;
   unsigned dead = 0;
+  const vdp::FPt fq = SPH ? load_fpt(T, qv) : vdp::FPt{};
   for (int j = lane, bit = 0; j < nfac; j += 32, ++bit) {
     const int* r = FR + 6 * j;
-    const int qf = r[5] & 3;
-    if (emit_simplex(T, r, W.id[j], set4(make_int4(-1, -1, -1, -1), qf, r[4]), round)) dead |= 1u << bit;
+    const int qf = rec_q(r[5]);
+    if (emit_simplex<D, SPH>(T, r, W.id[j], set4(make_int4(-1, -1, -1, -1), qf, r[4]), round, fq)) dead |= 1u << bit;
   }
   const int sweeps = (nfac * D / 2 + PER_SWEEP - 1) / PER_SWEEP;
   // the table is empty on entry (cleared when the warp starts, and after
@@ -1266,7 +1410,7 @@ __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __
       const int2* r2 = reinterpret_cast<const int2*>(FR + 6 * j);
       const int2 a = r2[0], b = r2[1], c = r2[2];
       const int r[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
-      const int qf = r[5] & 3;
+      const int qf = rec_q(r[5]);
       const int idj = W.id[j];
 #pragma unroll
       for (int g = 0; g < NV; ++g) {
@@ -1309,8 +1453,8 @@ __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __
 // Star of one winner, large case: every (facet, face) inserts its ridge into
 // an open-addressing table (two halves per ridge), then reads its partner.
 // A warp (BLOCK = false) or the whole block (k_commit_big) writes it.
-template <int D, bool BLOCK = false>
-__device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, int nfac, int round,
+template <int D, bool SPH, bool BLOCK = false>
+__device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, int nfac, int qv, int round,
                                int* R, int lane) {
   constexpr int NV = D + 1;
   const int G = BLOCK ? (int)blockDim.x : 32;
@@ -1327,7 +1471,7 @@ __device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, i
   for (int it = lane; it < nfac * NV; it += G) {
     const int j = it / NV, g = it - j * NV;
     const int* r = FR + 6 * j;
-    const int qf = r[5] & 3;
+    const int qf = rec_q(r[5]);
     if (g == qf) continue;
     int r0, r1;
     ridge_of<D>(r, g, qf, r0, r1);
@@ -1346,9 +1490,10 @@ __device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, i
     }
   }
   sync();
+  const vdp::FPt fq = SPH ? load_fpt(T, qv) : vdp::FPt{};
   for (int j = lane; j < nfac; j += G) {
     const int* r = FR + 6 * j;
-    const int qf = r[5] & 3;
+    const int qf = rec_q(r[5]);
     int4 nn = make_int4(-1, -1, -1, -1);
     nn = set4(nn, qf, r[4]);
     for (int g = 0; g < NV; ++g) {
@@ -1376,7 +1521,7 @@ __device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, i
       }
       nn = set4(nn, g, (ID[m] << 2) | (other & 3));
     }
-    emit_simplex(T, r, ID[j], nn, round);
+    emit_simplex<D, SPH>(T, r, ID[j], nn, round, fq);
   }
   sync();
 }
@@ -1391,11 +1536,11 @@ __device__ __forceinline__ void publish_shared_facets(const DevTree& T, int* F, 
   for (int j = lane; j < nfac; j += G) {
     const int o = F[6 * j + 4];
     if (o < 0 || bad_simp(T, o >> 2) || T.killed[o >> 2].x != round) continue;
-    const int kf = F[6 * j + 5], k = kf >> 2;
-    const int inner = (P[k] << 2) | (kf & 3);  // the removed simplex and its face on this facet
-    T.repl[inner] = (IDS[j] << 2) | (kf & 3);
+    const int kf = F[6 * j + 5];
+    const int inner = (P[rec_k(kf)] << 2) | rec_f(kf);  // the removed simplex and its face on this facet
+    T.repl[inner] = (IDS[j] << 2) | rec_q(kf);
     F[6 * j] = IDS[j];
-    F[6 * j + 1] = kf & 3;
+    F[6 * j + 1] = rec_q(kf);
     F[6 * j + 2] = -2;
   }
 }
@@ -1406,11 +1551,11 @@ __device__ __forceinline__ void publish_marked(const DevTree& T, int* F, const i
                                                unsigned dead, int lane) {
   for (int j = lane, bit = 0; j < nfac; j += 32, ++bit) {
     if (!((dead >> bit) & 1u)) continue;
-    const int kf = F[6 * j + 5], k = kf >> 2;
-    const int inner = (P[k] << 2) | (kf & 3);
-    T.repl[inner] = (IDS[j] << 2) | (kf & 3);
+    const int kf = F[6 * j + 5];
+    const int inner = (P[rec_k(kf)] << 2) | rec_f(kf);
+    T.repl[inner] = (IDS[j] << 2) | rec_q(kf);
     F[6 * j] = IDS[j];
-    F[6 * j + 1] = kf & 3;
+    F[6 * j + 1] = rec_q(kf);
     F[6 * j + 2] = -2;
   }
 }
@@ -1470,6 +1615,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
   int2 chunk = (MODE != 2 && gw < T.cap_wchunk) ? T.wchunk[gw] : make_int2(0, 0);
   const int nw = nblk * 4;
   const int lo = MODE == 2 ? T.ctr->win_lo : 0;
+  if (MODE == 2 && bid == 0 && threadIdx.x == 0) T.ctr->win_sph = lo;
   const int nin = MODE == 2 ? T.ctr->nwin : T.ctr->nwl[sin];
   const int* list = MODE == 2 ? T.win : T.wl[sin & 1];
   for (int it0 = lo + bid * 4 + wib; it0 < nin; it0 += 32 * nw) {
@@ -1582,7 +1728,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         // the other facets take the remaining cavity slots, then fresh ones
         for (int i = lane; i < ncav; i += 32) W.first[i] = 0x7fffffff;
         __syncwarp();
-        for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[__ldg(F + 6 * j + 5) >> 2], j);
+        for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[rec_k(__ldg(F + 6 * j + 5))], j);
         __syncwarp();
         int nfree = 0;  // cavity slots without an own facet, ranked
         for (int i0 = 0; i0 < ncav; i0 += 32) {
@@ -1598,7 +1744,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
           int id = 0;
           bool sec = false;
           if (j < nfac) {
-            const int k = __ldg(F + 6 * j + 5) >> 2;
+            const int k = rec_k(__ldg(F + 6 * j + 5));
             sec = W.first[k] != j;
             if (!sec) id = P[k];
           }
@@ -1616,7 +1762,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         // leftover cavity slots become holes pointing into the star
         for (int t = nsec + lane; t < nfree; t += 32)
           store_simplex(T, W.freeslot[t], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
-        dead = write_star<D>(T, W, F, nfac, cd.x, round, lane);
+        dead = write_star<D, D == 3 && MODE != 2>(T, W, F, nfac, cd.x, round, lane);
         small_star = true;
       } else {
         // large star (spilled search): plain slot assignment, ids in the
@@ -1635,7 +1781,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         IDS = ID;
         for (int i = nfac + lane; i < ncav; i += 32)
           store_simplex(T, P[i], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
-        write_star_big<D>(T, F, ID, nfac, round, P + kOffR, lane);
+        write_star_big<D, D == 3 && MODE != 2>(T, F, ID, nfac, cd.x, round, P + kOffR, lane);
       }
       if (MODE == 2) {
         // facets shared with another winner's cavity: publish this side's new
@@ -1645,6 +1791,8 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
           publish_marked(T, F, P, IDS, nfac, dead, lane);
         else
           publish_shared_facets<false>(T, F, P, IDS, nfac, round, lane);
+        if (D == 3)
+          for (int j = lane; j < nfac; j += 32) F[6 * j + 5] = IDS[j];  // for star_spheres
       }
       if (lane == 0) {
         write_hints_sampled<D>(T, cd.x, fq, id0, (unsigned)cd.z, hint_all);
@@ -1727,9 +1875,10 @@ __global__ void __launch_bounds__(512, 1) k_commit_big(DevTree T) {
     const int id0 = ID[0];
     for (int k = nfac + threadIdx.x; k < ncav; k += blockDim.x)
       store_simplex(T, P[k], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
-    write_star_big<D, true>(T, F, ID, nfac, round, P + kOffR, threadIdx.x);
+    write_star_big<D, D == 3, true>(T, F, ID, nfac, cd.x, round, P + kOffR, threadIdx.x);
     publish_shared_facets<true>(T, F, P, ID, nfac, round, threadIdx.x);
     if (threadIdx.x == 0) {
+      T.cinfo[c].y |= kSpheresDone;
       write_hints<D>(T, cd.x, load_fpt(T, cd.x), id0);
       T.cinfo[c].w = ST_DONE;
       T.act[par][cd.w].x = -1;
@@ -1746,13 +1895,34 @@ __global__ void __launch_bounds__(512, 1) k_commit_big(DevTree T) {
   }
 }
 
+// Stored spheres of the star of winner c (adjacent mode; a star of k_commit_big
+// has them already), by one warp.  Not in the commit half:
+// there the vertex loads and the sphere's arithmetic lie on every winner's path
+// (commit 7.1 -> 9.9 ms of the 1M-point build); the next kernel (k_reclaim, or
+// k_relocate after the last pass) has warps to spare for them.
+template <int D>
+__device__ __forceinline__ void star_spheres(const DevTree& T, int c, const int* F, int nfac, int lane) {
+  const int qv = T.cand[c].x;
+  const vdp::FPt fq = load_fpt(T, qv);
+  for (int j = lane; j < nfac; j += 32) {
+    const int id = F[6 * j + 5];
+    int4 v, n;
+    load_simplex(T, id, v, n);
+    const int r[4] = {v.x, v.y, v.z, v.w};
+    const int qf = v.x == qv ? 0 : (v.y == qv ? 1 : (v.z == qv ? 2 : 3));
+    store_sphere<D>(T, id, r, qf, fq);
+  }
+}
+
 // Adjacent mode, end of a round: a new simplex whose outer neighbour another
 // winner removed takes, as that neighbour, the other winner's new simplex on
-// the same facet.
+// the same facet.  The last pass's stars get their spheres.
+template <int D>
 __device__ __forceinline__ void fix_body(DevTree T, int bid, int nblk) {
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nw = nblk * (blockDim.x >> 5);
   const int n = T.ctr->nwin;
+  const int sph = T.ctr->win_sph;
   const long long nrepl = 4LL * T.cap_simp;
   // the last warps of the grid take the winners, so that in a small round the
   // first warps, which relocate the points, do not wait for this chain first
@@ -1772,6 +1942,7 @@ __device__ __forceinline__ void fix_body(DevTree T, int bid, int nblk) {
       }
       reinterpret_cast<int*>(T.simp + id)[4 + g] = T.repl[o];
     }
+    if (D == 3 && it >= sph && !(info.y & kSpheresDone)) star_spheres<D>(T, c, F, nfac, lane);
   }
 }
 
@@ -1817,15 +1988,27 @@ __device__ __forceinline__ void reclaim_body(DevTree T, int pass, int adjacent, 
       T.wl[sout & 1][k] = c;
     }
   }
+  if (D == 3 && adjacent) {
+    // spheres of the previous pass's stars, by the last warps first
+    const int n = T.ctr->nwin;
+    for (int i = T.ctr->win_sph + nw - 1 - (bid * 4 + wib); i < n; i += nw) {
+      const int c = T.win[i];
+      const int4 info = T.cinfo[c];
+      int *P, *F, ncav, nfac;
+      bool big;
+      cand_lists(T, info, P, F, ncav, nfac, big);
+      if (info.w == ST_DONE && !(info.y & kSpheresDone)) star_spheres<D>(T, c, F, nfac, lane);
+    }
+  }
 }
 template <int D>
-__global__ void __launch_bounds__(128) k_reclaim(DevTree T, int pass, int adjacent) { reclaim_body<D>(T, pass, adjacent, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(128, 6) k_reclaim(DevTree T, int pass, int adjacent) { reclaim_body<D>(T, pass, adjacent, blockIdx.x, gridDim.x); }
 
 template <int D>
 __device__ __forceinline__ void relocate_body(DevTree T, int bid, int nblk) {
   // adjacent mode: first link the stars of winners that share facets (the
   // walks below stay inside stars, so they do not need those links)
-  fix_body(T, bid, nblk);
+  fix_body<D>(T, bid, nblk);
   const int round = T.ctr->round;
   constexpr int NV = D + 1;
   const int par = round & 1;
@@ -2099,14 +2282,15 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
   int4 v0, n0;
   load_simplex(T, start, v0, n0);
   unsigned ntests = 0;
-  const CavStore S{C.cav, C.cv, C.cn, C.hkey, C.fr, MAXC, MAXF, HS};
-  cavity_search<D, 0>(T, S, C.ctl, lane, start, v0, n0, vid, fq, tl, perr, ntests);
-  if (C.ctl.flags) {  // too large for the warp: the rounds insert it
+  if (lane == 0) C.st.clear();
+  __syncwarp();
+  const CavStore S{C.cav, C.cn, C.hkey, F, C.und, &C.st, MAXC, MAXF, HS};
+  const Region rg = cavity_search<D, 0>(T, S, lane, start, n0, vid, fq, tl, perr, ntests);
+  if (rg.over) {  // too large for the warp: the rounds insert it
     if (lane == 0) ctr->single = -1;
     return;
   }
-  const int ncav = C.ctl.ncav, nfac = C.ctl.nfac;
-  expand_facets(C.fr, C.cv, nfac, vid, F, lane);
+  const int ncav = rg.ncav, nfac = rg.nfac;
   for (int i = lane; i < HR; i += 32) {
     W.rk[i] = ~0ull;
     W.ra[i] = -1;
@@ -2115,7 +2299,7 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
   __syncwarp();
   // slots: the first facet of cavity simplex k takes k's slot, the others
   // the cavity slots left over, then fresh ones
-  for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[F[6 * j + 5] >> 2], j);
+  for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[rec_k(F[6 * j + 5])], j);
   __syncwarp();
   int nfree = 0;
   for (int i0 = 0; i0 < ncav; i0 += 32) {
@@ -2142,7 +2326,7 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
     int id = 0;
     bool sec = false;
     if (j < nfac) {
-      const int k = F[6 * j + 5] >> 2;
+      const int k = rec_k(F[6 * j + 5]);
       sec = W.first[k] != j;
       if (!sec) id = C.cav[k];
     }
@@ -2159,7 +2343,8 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
   for (int t = nsec + lane; t < nfree; t += 32)
     store_simplex(T, W.freeslot[t], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
   // no slot carries round -2 in `killed`, so every outer neighbour is repointed
-  write_star<D>(T, W, F, nfac, vid, -2, lane);
+  write_star<D, D == 3>(T, W, F, nfac, vid, -2, lane);
+  C.st.merge<D>(tl, perr, ntests, lane);
   if (perr) set_error(ctr, E_PRECISION);
   flush_tally(ctr, tl, ntests, 0);
   if (lane == 0) {
@@ -2514,6 +2699,12 @@ __global__ void __launch_bounds__(kSeedThreads, 1) k_seed(DevTree T, int npts, i
       gn = set4(gn, j, c < 0 ? -1 : (mark[c >> 2] << 2) | (c & 3));
     }
     store_simplex(T, mark[s], gv, gn);
+    if (D == 3) {
+      vdp::FPt lv[NV];
+      for (int j = 0; j < NV; ++j) lv[j] = fp[get4(v, j)];
+      const vdp::Sph c = vdp::sphere_of<D>(lv);
+      *reinterpret_cast<float4*>(T.sph + mark[s]) = make_float4(c.x, c.y, c.z, c.w);  // mark[s] < nlive <= cap_simp
+    }
     for (int j = 0; j < NV; ++j) {
       const int l = get4(v, j);
       if (l >= NV) write_hints<D>(T, gid[l], fp[l], mark[s]);
@@ -2606,7 +2797,7 @@ void round_impl(const DevTree& T, const Launch& L, const Tuning& tu, const Feed&
   for (int p = 0; p < tu.passes; ++p) {
     const int last = p == tu.passes - 1;
     if (p > 0) {
-      // reclaim (40 registers, no shared memory) runs twice the search's warps
+      // reclaim (73 registers, no shared memory) runs twice the search's warps
       k_reclaim<D><<<L.warps / 2, 128, 0, L.stream>>>(T, p, tu.adjacent);
       mark(KT_RECLAIM);
     }
@@ -2751,6 +2942,10 @@ int launch_small_rounds(const DevTree& T, cudaStream_t stream, int dim, const Tu
   }
   note_launches(1);
   return E_OK;
+}
+
+int search_chunk_ints(int dim) {
+  return dim == 3 ? region_ints(Cap<3>::MAXC, Cap<3>::MAXF) : region_ints(Cap<2>::MAXC, Cap<2>::MAXF);
 }
 
 int seed_max_points(int dim) { return dim == 3 ? SeedCap<3>::P - 4 : SeedCap<2>::P - 3; }

@@ -309,7 +309,7 @@ int ensure_simplices(vd_tree* t, int64_t want) {
   want = std::max(want, cap + cap / 2);
   if (want > (int64_t(1) << 29)) return vd::E_NOMEM;  // neighbour codes use 30 bits
   int64_t used = t->hctr->nsimp;
-  int64_t c[7] = {cap, cap, cap, cap, cap, cap, cap};
+  int64_t c[8] = {cap, cap, cap, cap, cap, cap, cap, cap};
   int rc = vd::E_OK;
   rc |= grow(&t->T.simp, &c[0], want, used, 0xff, t->stream);
   rc |= grow(&t->T.vote, &c[1], want, used, 0xff, t->stream);
@@ -318,6 +318,7 @@ int ensure_simplices(vd_tree* t, int64_t want) {
   rc |= grow(&t->T.claim_n, &c[4], want, used, 0xff, t->stream);
   rc |= grow(&t->T.killed, &c[5], want, used, 0xff, t->stream);
   rc |= grow(&t->T.touched, &c[6], want, used, 0xff, t->stream);
+  if (t->dim == 3) rc |= grow(&t->T.sph, &c[7], want, used, -1, t->stream);  // written with every simplex
   int64_t cr = 4 * cap;  // read only where written in the same round
   rc |= grow(&t->T.repl, &cr, 4 * want, 0, -1, t->stream);
   if (rc) return vd::E_NOMEM;
@@ -360,8 +361,12 @@ int ensure_points(vd_tree* t, int64_t n_new) {
     t->cap_act = c;
     t->T.cap_cand = (int)c;
   }
+  // room for eight spilled searches and a chunk of every warp that can search
+  // in one round, or what a round of n_new points needs
+  const int64_t warps = std::min<int64_t>(n_new, (int64_t)t->sms * kMaxWarpsPerSm);
   const int64_t pool_want = std::min<int64_t>(
-      std::max<int64_t>((t->dim == 3 ? 48 : 24) * std::max<int64_t>(n_new, 1024), 8 * 360448 + 64),
+      std::max<int64_t>((t->dim == 3 ? 48 : 24) * std::max<int64_t>(n_new, 1024),
+                        8 * 360448 + 64 + warps * vd::search_chunk_ints(t->dim)),
       0x7fffffffLL);
   if (pool_want > t->T.cap_pool) {
     dfree(t->T.pool);
@@ -399,6 +404,7 @@ void release(vd_tree* t) {
   dfree(t->T.pts);
   dfree(t->T.ptf);
   dfree(t->T.simp);
+  dfree(t->T.sph);
   dfree(t->T.vote);
   dfree(t->T.thin);
   dfree(t->T.claim_c);
@@ -630,6 +636,8 @@ int set_geometry_sets(vd_tree* t, int nsets, const double* c, const double* rb, 
   if (used > 0) cudaMemsetAsync(t->T.simp, 0xff, sizeof(vd::Simplex) * used, t->stream);
   t->simp_hwm = nsets;
   cudaMemcpyAsync(t->T.simp, roots.data(), sizeof(vd::Simplex) * nsets, cudaMemcpyHostToDevice, t->stream);
+  if (dim == 3)  // NaN: the roots have no stored sphere
+    cudaMemsetAsync(t->T.sph, 0xff, sizeof(vdp::Sph) * nsets, t->stream);
   t->nverts = ns;
   t->inserted = 0;
   t->round_base = t->round;

@@ -12,6 +12,8 @@
 //                 opposite v[f], or -1 on the super-simplex hull; a dead slot
 //                 has v[0] = -1 and n[0] pointing at a simplex of the star that
 //                 replaced it.  32 B = one sector.
+//   sph[s]        stored circumsphere of s (3D), the first tier of the conflict
+//                 test: centre and squared radius, 16 B (vdp::Sph)
 //   vote[s]       epoch|priority of the lowest-priority uninserted point inside s
 //   thin[s]       epoch|priority of the lowest candidate whose simplex is s or
 //                 a face neighbour of s (cheap pre-selection before any search)
@@ -103,6 +105,7 @@ struct Counters {
   int feed_lo, feed_hi;             // range of `order` activated this round
   int round;                        // round being run (advanced by k_plan)
   int nwin, win_lo;                 // winners of the round (adjacent mode), first of the pass
+  int win_sph;                      // first winner whose star has no stored spheres yet
   int max_levels;                   // deepest cavity search (breadth-first levels)
   // grid barrier and loop decision of the small-round kernel
   unsigned bar_count, bar_gen;
@@ -147,6 +150,7 @@ struct DevTree {
   vdp::VPt* pts;
   vdp::FPt* ptf;      // the same coordinates split into f32 hi/lo pairs
   Simplex* simp;
+  vdp::Sph* sph;
   unsigned long long* vote;
   unsigned long long* thin;
   unsigned long long* claim_c;
@@ -295,6 +299,8 @@ struct Prof {
   int type[kMax];
   int n;
 };
+// Pool ints a warp of the region search takes at least at a time.
+int search_chunk_ints(int dim);
 // Kernel attributes the rounds need (shared-memory size); once per device
 // before the first round or capture.
 int prepare_round_kernels();

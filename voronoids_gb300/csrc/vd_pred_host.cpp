@@ -138,3 +138,20 @@ int vdh_exit_face_hl(int dim, const double* pts, unsigned mask, int strict, int*
 }
 
 }  // extern "C"
+
+extern "C" {
+
+// Stored-sphere tier alone: +1 inside, -1 outside (certain), 0 undecided.
+// `rot` rotates the simplex's points, so that each can be the base.
+int vdh_sphere_side(int dim, const double* pts, int rot) {
+  vdp::FPt f[4];
+  for (int i = 0; i <= dim; ++i) {
+    const double* p = pts + 3 * ((i + rot) % (dim + 1));
+    f[i] = vdp::split_point(p[0], p[1], p[2]);
+  }
+  const int k = dim + 1;
+  const vdp::FPt fq = vdp::split_point(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]);
+  return dim == 3 ? vdp::sphere_side<3>(vdp::sphere_of<3>(f), fq) : vdp::sphere_side<2>(vdp::sphere_of<2>(f), fq);
+}
+
+}  // extern "C"

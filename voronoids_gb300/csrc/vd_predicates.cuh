@@ -1018,6 +1018,154 @@ VDP_HD int insphere_hl(const FPt* v, const FPt& q) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Sphere tier.  A simplex that stays is tested against a few query points, so
+// its circumsphere is worth storing: centre and squared radius in 16 bytes,
+// against the 128 bytes of its vertices' split records.  The stored centre c'
+// is any float point near the true centre c; what makes the test certain is a
+// bound E on |e|, e = c - c', found after the fact from the distances of the
+// vertices to c' itself:
+//   r_i^2 - r_0^2 = 2 (v_i - v_0) . e            (i = 1..D), so
+//   |e| <= sum_i |r_i^2 - r_0^2| |d_j x d_k| / (2 |det d|)
+// and, since the power of q is |q - c'|^2 - r_0^2 - 2 e . (q - v_0),
+//   |q - c'| > r_0 + 2E  =>  outside,     |q - c'| < r_0 - 2E  =>  inside.
+// Rounding (u = 2^-24, L = largest |difference| between vertices, M = largest
+// |coordinate|; the tier is used only for M <= 2^20 L, |c'| <= 2^21 r_0,
+// 2^-25 <= L <= 2^20 and |det| >= 2^-14 L^D, so that nothing under- or
+// overflows):
+//   a difference of vertices is within 3uL, a component of d_j x d_k within
+//   15uL^2 (its 1-norm within 2^-16 L^2), det within 128u L^D <= |det| / 8;
+//   a component of q - c' is within 2u |q - c'| + u r_0 / 4 (the split of q
+//   costs u^2 |q| <= u^2 (2^21 r_0 + |q - c'|)), so a squared distance is
+//   within 8u max(|q - c'|^2, r_0^2);
+//   hence the relative half-width of the band around r_0^2 in which q is
+//   undecided: 4.25 E / r_0 + 20u (E <= r_0 / 16) + 2^-19 for the four low
+//   mantissa bits of r_0^2, which hold the width: the band is
+//   r_0^2 (1 +- 2^-(2 + bits)).
+// A simplex that the tier cannot serve has r_0^2 = NaN, and a point whose split
+// is not accurate carries a NaN (hw): every comparison then fails.
+// tests/test_sphere_tier.py holds certain answers to the exact sign.
+// ---------------------------------------------------------------------------
+struct alignas(16) Sph {
+  float x, y, z, w;
+};
+VDP_HD float bits_f32(uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __uint_as_float(b);
+#else
+  float f;
+  memcpy(&f, &b, 4);
+  return f;
+#endif
+}
+VDP_HD uint32_t f32_bits(float f) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(f);
+#else
+  uint32_t b;
+  memcpy(&b, &f, 4);
+  return b;
+#endif
+}
+
+// Squared distance of p to the stored centre (see above); NaN if p's split is
+// not accurate.
+template <int D>
+VDP_HD float sphere_dist2(float cx, float cy, float cz, const FPt& p) {
+  const float x = fadd_rn(fsub_rn(p.hx, cx), p.lx), y = fadd_rn(fsub_rn(p.hy, cy), p.ly);
+  float s = ffma(y, y, fmulr(x, x));
+  if (D == 3) {
+    const float z = fadd_rn(fsub_rn(p.hz, cz), p.lz);
+    s = ffma(z, z, s);
+  }
+  return s + p.hw;
+}
+
+// Stored circumsphere of the simplex v[0..D].
+template <int D>
+VDP_HD Sph sphere_of(const FPt* v) {
+  constexpr int NV = D + 1;
+  Sph out{0.0f, 0.0f, 0.0f, bits_f32(0x7fc00000u)};
+  float x[D], y[D], z[D], M = 0.0f, L = 0.0f, flag = v[0].hw;
+  for (int i = 0; i < NV; ++i) M = fmaxf(M, fmaxf(fabsf(v[i].hx), fmaxf(fabsf(v[i].hy), fabsf(v[i].hz))));
+  for (int i = 0; i < D; ++i) {
+    x[i] = hl_diff(v[i + 1].hx, v[i + 1].lx, v[0].hx, v[0].lx);
+    y[i] = hl_diff(v[i + 1].hy, v[i + 1].ly, v[0].hy, v[0].ly);
+    z[i] = D == 3 ? hl_diff(v[i + 1].hz, v[i + 1].lz, v[0].hz, v[0].lz) : 0.0f;
+    L = fmaxf(L, fmaxf(fabsf(x[i]), fmaxf(fabsf(y[i]), fabsf(z[i]))));
+    flag += v[i + 1].hw;
+  }
+  L += flag;
+  if (!(L >= 2.98023223876953125e-8f && L <= 1048576.0f && M <= 1048576.0f * L)) return out;
+  // n[i]: 1-norm of the cofactor row that goes with d_i
+  float det, n[D], ox, oy, oz = 0.0f, floor_det;
+  const float L2 = L * L;
+  if (D == 3) {
+    const float px = ffma(y[1], z[2 % D], -(z[1] * y[2 % D])), py = ffma(z[1], x[2 % D], -(x[1] * z[2 % D])),
+                pz = ffma(x[1], y[2 % D], -(y[1] * x[2 % D]));
+    const float qx = ffma(y[2 % D], z[0], -(z[2 % D] * y[0])), qy = ffma(z[2 % D], x[0], -(x[2 % D] * z[0])),
+                qz = ffma(x[2 % D], y[0], -(y[2 % D] * x[0]));
+    const float rx = ffma(y[0], z[1], -(z[0] * y[1])), ry = ffma(z[0], x[1], -(x[0] * z[1])),
+                rz = ffma(x[0], y[1], -(y[0] * x[1]));
+    det = ffma(z[0], pz, ffma(y[0], py, x[0] * px));
+    const float a2 = ffma(z[0], z[0], ffma(y[0], y[0], x[0] * x[0]));
+    const float b2 = ffma(z[1], z[1], ffma(y[1], y[1], x[1] * x[1]));
+    const float c2 = ffma(z[2 % D], z[2 % D], ffma(y[2 % D], y[2 % D], x[2 % D] * x[2 % D]));
+    const float h = 0.5f / det;
+    ox = (a2 * px + b2 * qx + c2 * rx) * h;
+    oy = (a2 * py + b2 * qy + c2 * ry) * h;
+    oz = (a2 * pz + b2 * qz + c2 * rz) * h;
+    n[0] = fabsf(px) + fabsf(py) + fabsf(pz);
+    n[1] = fabsf(qx) + fabsf(qy) + fabsf(qz);
+    n[2 % D] = fabsf(rx) + fabsf(ry) + fabsf(rz);
+    floor_det = 6.103515625e-5f * (L2 * L);  // 2^-14 L^3
+  } else {
+    det = ffma(x[0], y[1], -(y[0] * x[1]));
+    const float a2 = ffma(y[0], y[0], x[0] * x[0]), b2 = ffma(y[1], y[1], x[1] * x[1]);
+    const float h = 0.5f / det;
+    ox = (a2 * y[1] - b2 * y[0]) * h;
+    oy = (b2 * x[0] - a2 * x[1]) * h;
+    n[0] = fabsf(x[1]) + fabsf(y[1]);
+    n[1] = fabsf(x[0]) + fabsf(y[0]);
+    floor_det = 6.103515625e-5f * L2;  // 2^-14 L^2
+  }
+  if (!(fabsf(det) >= floor_det)) return out;
+  const float cx = v[0].hx + (v[0].lx + ox), cy = v[0].hy + (v[0].ly + oy),
+              cz = D == 3 ? v[0].hz + (v[0].lz + oz) : 0.0f;
+  const float r0 = sphere_dist2<D>(cx, cy, cz, v[0]);
+  float r[D], rmax = r0;
+  for (int i = 0; i < D; ++i) {
+    r[i] = sphere_dist2<D>(cx, cy, cz, v[i + 1]);
+    rmax = fmaxf(rmax, r[i]);
+  }
+  const float slack = 1.1e-6f * rmax;  // 18u: both squared distances and their difference
+  const float nslack = D == 3 ? 1.52587890625e-5f * L2 : 1.52587890625e-5f * L;  // 2^-16
+  float e = 0.0f;
+  for (int i = 0; i < D; ++i) e += (fabsf(r[i] - r0) + slack) * (n[i] + nslack);
+  e = 0.6f * e / fabsf(det);  // 1 / (2 * 7/8) and the rounding of this sum
+  const float width = 4.6f * e / sqrtf(r0) + 4.2e-6f;  // 4.25 E / r_0 + 20u + 2^-19, rounded up
+  const float cm = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz)));
+  if (!(width < 0.25f && r0 <= 1.2089258196146292e24f && cm * cm <= 4.398046511104e12f * r0)) return out;
+  // width < 2^(ex + 1) with ex the exponent of width: bits = -3 - ex, at most 15
+  const int ex = (int)(f32_bits(width) >> 23) - 127;
+  const int code = -3 - ex < 15 ? -3 - ex : 15;
+  out.x = cx;
+  out.y = cy;
+  out.z = cz;
+  out.w = bits_f32((f32_bits(r0) & ~15u) | (uint32_t)code);
+  return out;
+}
+
+// Side of q: +1 inside, -1 outside (both certain), 0 undecided.
+template <int D>
+VDP_HD int sphere_side(const Sph& c, const FPt& q) {
+  const float s = sphere_dist2<D>(c.x, c.y, c.z, q);
+  const uint32_t b = f32_bits(c.w);
+  const float w = bits_f32(b & ~15u);
+  const float t = bits_f32((125u - (b & 15u)) << 23);  // 2^-(2 + bits)
+  return s > ffma(w, t, w) ? -1 : (s < ffma(w, -t, w) ? 1 : 0);
+}
+
 // The FP64 and exact tiers of in_conflict (used when the split tier is undecided).
 template <int D, int XT = 1>
 VDP_HD bool in_conflict_64(const VPt* p, const int* key, const VPt& q, int qkey, Tally& t, int& err) {

@@ -28,9 +28,9 @@
 
 namespace {
 
-// Estimated device bytes of a request, with 1.5x slack: simplex slots (3D
-// 7.6, 2D 2.3 per point, 92 B each: record, claims, marks, star links) and
-// per-point records, work lists and edge scratch (about 520 B in 3D, 250 B
+// Estimated device bytes of a request, with slack (3D 1.4x, 2D 1.5x): simplex
+// slots (3D 7.6 per point of 108 B, 2D 2.3 of 92 B: record, stored sphere in
+// 3D, claims, marks, star links) and per-point records, work lists and edge scratch (about 520 B in 3D, 250 B
 // in 2D).
 int64_t estimate_bytes(int dim, int64_t n) { return (dim == 3 ? 1850 : 700) * std::max<int64_t>(n, 1) + 4096; }
 
