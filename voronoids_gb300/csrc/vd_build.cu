@@ -2368,101 +2368,129 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
 // the super simplex's star, so a device-wide round inserts one or a few points
 // for about ten dependent kernel launches.  Here one 512-thread block inserts
 // the first priority levels (Bowyer-Watson in the reference's sense,
-// src/delaunay_tree.rs:125-211, one point at a time):
-//   1. every live simplex is tested against the point (exact, perturbed
-//      conflict test keyed by the global vertex ids, as in the rounds), so no
-//      point location is needed;
+// src/delaunay_tree.rs:125-211, one point at a time), three barriers a point:
+//   1. every slot is tested against the point, so no point location is needed:
+//      by its stored sphere, or by the vertices (exact, perturbed, keyed by the
+//      global vertex ids, as in the rounds) where that cannot decide; a point
+//      equal to a vertex is a duplicate.  The simplices of the last star are
+//      tested by warps of their own, which make their spheres first, so that
+//      this long chain runs beside the scan of the slots and not in each warp
+//      that meets one of them;
 //   2. the faces of the conflict region whose neighbour is outside it are the
-//      boundary facets; no conflict region means the point duplicates a vertex;
+//      boundary facets, and each enters the faces through the new point into a
+//      ridge table;
 //   3. each facet gets a new simplex (a region slot first, then a fresh slot)
-//      with its outer link, and the faces through the new point are paired
-//      through a ridge table.
+//      with its outer link and its partners from the ridge table, and the outer
+//      neighbour is relinked.
 // The triangulation is unique, so any insertion order gives the one the
 // rounds would build.  The tree in global memory is written only at the end,
 // compacted (live simplices in slots 0..m-1) with the location hints of every
 // point; when any capacity below would be exceeded the kernel writes nothing
 // and the rounds insert these points as usual.
+//
+// Slots are 32 bytes (16-bit local vertex ids and links, sphere), so a block
+// holds 644 points in 3D and 1,665 in 2D.  What bounds it is the chain of the
+// three steps: about 4,000 cycles a point in 3D (369 points: 0.76 ms; the form
+// with vertex tests of every slot, 32-byte links and six barriers took 0.51 ms
+// for 144 points, this one 0.29 ms).
 constexpr int kSeedThreads = 512;
+// S slots, P vertices (super vertices too), F facets and region slots (one
+// thread each), H ridge table entries.
 template <int D>
 struct SeedCap;
 template <>
 struct SeedCap<3> {
-  static constexpr int S = 2560, P = 324, C = 1024, F = 1024, H = 4096, DUP = 64;
+  static constexpr int S = 4864, P = 648, F = kSeedThreads, H = 2048;
 };
 template <>
 struct SeedCap<2> {
-  static constexpr int S = 2560, P = 644, C = 1024, F = 1024, H = 4096, DUP = 64;
+  static constexpr int S = 3456, P = 1668, F = kSeedThreads, H = 2048;
 };
-// Shared-memory layout of k_seed (bytes), in this order: simplex vertices and
-// neighbour codes (local ids), point records and global ids, cavity marks,
-// cavity, facets (new vertices, outer code, position of the new point), ridge
-// table (keys, first and second half), flags of inserted points, duplicates.
+// Shared-memory layout of k_seed (bytes), in this order: spheres, vertices and
+// links of the slots, point records and global ids, facets (new vertices, outer
+// code, position of the new point), ridge table (keys, first and second half),
+// region, slots of the last star, marks, duplicates, a slot per vertex.
 template <int D>
 constexpr size_t seed_smem() {
   using C = SeedCap<D>;
-  return (size_t)C::S * 32 + (size_t)C::P * (sizeof(vdp::FPt) + 4) + (size_t)C::S * 4 + (size_t)C::C * 4 +
-         (size_t)C::F * 24 + (size_t)C::H * 16 + (size_t)C::P * 4 + (size_t)C::DUP * 8;
+  return (size_t)C::S * (sizeof(vdp::Sph) + 8 + 8) + (size_t)C::P * (sizeof(vdp::FPt) + 4) + (size_t)C::F * (8 + 2 + 2) +
+         (size_t)C::H * (4 + 2 + 2) + (size_t)C::F * 2 * 2 + (size_t)C::S * 2 + (size_t)C::P * 2 * 2;
 }
-__device__ __forceinline__ unsigned seed_hash(int r0, int r1, int H) {
-  return ((((unsigned)r0 * 0x9E3779B1u) ^ ((unsigned)r1 * 0x85EBCA77u)) >> 12) & (unsigned)(H - 1);
+static_assert(seed_smem<3>() <= 232448 - 1024 && seed_smem<2>() <= 232448 - 1024, "a block's shared memory");
+static_assert(SeedCap<3>::P <= 1024 && SeedCap<2>::P < 2048 && SeedCap<3>::P % 2 == 0 && SeedCap<2>::P % 2 == 0 &&
+                  SeedCap<3>::S * 4 < 0xffff && SeedCap<2>::S * 4 < 0xffff,
+              "16-bit links, ridge keys of 20 bits");
+__device__ __forceinline__ int get4(const ushort4& a, int i) {
+  return i == 0 ? a.x : (i == 1 ? a.y : (i == 2 ? a.z : a.w));
 }
-// Slot of the key (epoch, r0, r1) in the ridge table, -1 if absent.
-__device__ __forceinline__ int seed_find(const unsigned long long* hk, int H, unsigned long long key, int r0, int r1) {
-  unsigned h = seed_hash(r0, r1, H);
-  for (int probe = 0; probe < H; ++probe, h = (h + 1) & (unsigned)(H - 1)) {
-    const unsigned long long k = hk[h];
-    if (k == key) return (int)h;
-    if ((k >> 32) != (key >> 32)) return -1;  // an entry of an earlier point: the key is not there
-  }
-  return -1;
+// Four packed local vertices with position f replaced by l.
+__device__ __forceinline__ unsigned long long seed_replace(unsigned long long v, int f, int l) {
+  return (v & ~(0xffffull << (16 * f))) | ((unsigned long long)(unsigned)l << (16 * f));
+}
+// Ridge key: insertion number and the ridge's local vertices, those of v at
+// the positions other than gf and qf (3D two, 2D one).
+template <int D>
+__device__ __forceinline__ unsigned seed_key(int epoch, unsigned long long v, int gf, int qf) {
+  const unsigned rem = ((1u << (D + 1)) - 1u) & ~(1u << gf) & ~(1u << qf);
+  const unsigned a = (unsigned)(v >> (16 * (__ffs((int)rem) - 1))) & 0xffffu;
+  if (D == 2) return ((unsigned)epoch << 20) | a;
+  const unsigned b = (unsigned)(v >> (16 * (31 - __clz((int)rem)))) & 0xffffu;
+  return ((unsigned)epoch << 20) | (min(a, b) << 10) | max(a, b);
+}
+__device__ __forceinline__ unsigned seed_hash(unsigned key, int H) {
+  return ((key * 0x9E3779B1u) >> 12) & (unsigned)(H - 1);
 }
 
 template <int D>
 __global__ void __launch_bounds__(kSeedThreads, 1) k_seed(DevTree T, int npts, int nlev, unsigned long long seed) {
   using C = SeedCap<D>;
   constexpr int NV = D + 1;
+  constexpr unsigned short NONE = 0xffff;
+  constexpr float kNoSphere = -1.0f;  // sph[].w of a dead slot and of one in `fresh` (a sphere's is positive or NaN)
   extern __shared__ __align__(16) unsigned char seed_sm[];
-  int4* sv = reinterpret_cast<int4*>(seed_sm);
-  int4* sn = sv + C::S;
+  float4* sph = reinterpret_cast<float4*>(seed_sm);
+  ushort4* sv = reinterpret_cast<ushort4*>(sph + C::S);
+  ushort4* sn = sv + C::S;
   vdp::FPt* fp = reinterpret_cast<vdp::FPt*>(sn + C::S);
   int* gid = reinterpret_cast<int*>(fp + C::P);
-  int* mark = gid + C::P;
-  int* cav = mark + C::S;
-  int4* fnv = reinterpret_cast<int4*>(cav + C::C);
-  int* fcode = reinterpret_cast<int*>(fnv + C::F);
-  int* fqf = fcode + C::F;
-  unsigned long long* hk = reinterpret_cast<unsigned long long*>(fqf + C::F);
-  int* ha = reinterpret_cast<int*>(hk + C::H);
-  int* hb = ha + C::H;
-  int* ins = hb + C::H;
-  int2* dl = reinterpret_cast<int2*>(ins + C::P);
-  __shared__ int s_ns, s_ncav, s_nfac, s_abort, s_ndup, s_dupof, s_nins;
-  __shared__ unsigned long long s_created, s_killed;
-  __shared__ int s_maxc, s_maxf, s_holes;
+  ushort4* fnv = reinterpret_cast<ushort4*>(gid + C::P);
+  unsigned* hk = reinterpret_cast<unsigned*>(fnv + C::F);
+  unsigned short* fcode = reinterpret_cast<unsigned short*>(hk + C::H);
+  unsigned short* fqf = fcode + C::F;
+  unsigned short* ha = fqf + C::F;
+  unsigned short* hb = ha + C::H;
+  unsigned short* cav = hb + C::H;
+  unsigned short* fresh = cav + C::F;
+  unsigned short* mark = fresh + C::F;
+  unsigned short* dup = mark + C::S;  // 1 + the local vertex a point equals, 0 if none
+  unsigned short* home = dup + C::P;  // a slot with the vertex
+  __shared__ int s_ncav[2], s_nfac[2], s_dup[2], s_abort, s_ndup;
   const int tid = threadIdx.x;
   const SetGeo& g = T.sets[0];
-  if (T.nsets != 1 || npts < 1 || npts + NV > C::P || npts > C::C || npts > C::S) return;
+  if (T.nsets != 1 || npts < 1 || npts + NV > C::P || npts > C::H) return;
   // start: the super simplex (local vertices 0..D) and the points of the
   // levels in priority order (local vertex NV + k is the k-th lowest), so that
   // of equal points the one with the lowest priority is inserted and the
   // others are its duplicates, as in the rounds
-  for (int i = tid; i < npts; i += kSeedThreads) {
-    const int v = T.order[i];
-    mark[i] = v;
-    cav[i] = (int)priority((uint32_t)v, seed);
-  }
-  for (int i = tid; i < C::H; i += kSeedThreads) hk[i] = 0ull;
-  __syncthreads();
-  for (int i = tid; i < npts; i += kSeedThreads) {
-    const unsigned pr = (unsigned)cav[i];
-    int rank = 0;
-    for (int j = 0; j < npts; ++j) rank += (unsigned)cav[j] < pr ? 1 : 0;
-    const int v = mark[i];
-    const bool bad = bad_vert(T, v);
-    if (bad) set_error(T.ctr, E_INTERNAL);
-    gid[NV + rank] = bad ? 0 : v;
-    fp[NV + rank] = load_fpt(T, bad ? 0 : v);
-    ins[NV + rank] = 0;
+  {
+    int* tv = reinterpret_cast<int*>(sph);  // vertex, priority: the spheres' space is free yet
+    unsigned* tp = reinterpret_cast<unsigned*>(tv + C::P);
+    for (int i = tid; i < npts; i += kSeedThreads) {
+      const int v = T.order[i];
+      tv[i] = v;
+      tp[i] = priority((uint32_t)v, seed);
+    }
+    __syncthreads();
+    for (int i = tid; i < npts; i += kSeedThreads) {
+      const unsigned pr = tp[i];
+      int rank = 0;
+      for (int j = 0; j < npts; ++j) rank += tp[j] < pr ? 1 : 0;
+      const int v = tv[i];
+      const bool bad = bad_vert(T, v);
+      if (bad) set_error(T.ctr, E_INTERNAL);
+      gid[NV + rank] = bad ? 0 : v;
+      fp[NV + rank] = load_fpt(T, bad ? 0 : v);
+    }
   }
   for (int l = tid; l < NV; l += kSeedThreads) {
     const int v = g.sup[l];
@@ -2470,202 +2498,224 @@ __global__ void __launch_bounds__(kSeedThreads, 1) k_seed(DevTree T, int npts, i
     if (bad) set_error(T.ctr, E_INTERNAL);
     gid[l] = bad ? 0 : v;
     fp[l] = load_fpt(T, bad ? 0 : v);
-    ins[l] = 1;
   }
-  __syncthreads();
   for (int i = tid; i < C::S; i += kSeedThreads) mark[i] = 0;
+  for (int i = tid; i < C::P; i += kSeedThreads) dup[i] = 0;
+  for (int i = tid; i < C::H; i += kSeedThreads) hk[i] = 0u;
+  __syncthreads();
   if (tid == 0) {
-    sv[0] = D == 3 ? make_int4(0, 1, 2, 3) : make_int4(0, 1, 2, -1);
-    sn[0] = make_int4(-1, -1, -1, -1);
-    s_ns = 1;
-    s_ncav = s_nfac = s_abort = s_ndup = s_nins = 0;
-    s_created = s_killed = 0ull;
-    s_maxc = s_maxf = s_holes = 0;
+    sv[0] = make_ushort4(0, 1, 2, D == 3 ? 3 : NONE);
+    sn[0] = make_ushort4(NONE, NONE, NONE, NONE);
+    sph[0] = make_float4(0.0f, 0.0f, 0.0f, NAN);
+    s_ncav[0] = s_nfac[0] = s_abort = s_ndup = 0;
+    s_dup[0] = -1;
   }
   __syncthreads();
   vdp::Tally tl = {0, 0, 0, 0};
   int perr = 0;
   unsigned ntests = 0;
+  // the same in every thread: slots in use, slots of the last star, sums
+  int ns = 1, nfresh = 0, nins = 0, ncreated = 0, nkilled = 0, maxc = 0, maxf = 0, holes = 0;
+  bool abort = false;
   for (int p = 0; p < npts; ++p) {
-    const int ql = NV + p, qv = gid[ql];
+    const int ql = NV + p, qv = gid[ql], par = p & 1;
     const vdp::FPt fq = fp[ql];
-    const int ns = s_ns;
-    // 0. a point equal to an inserted vertex is skipped and recorded, as the
-    // rounds do before any search (its conflict region need not be empty:
-    // the perturbation of an equal vertex with a larger id puts it inside)
-    if (tid == 0) s_dupof = -1;
-    __syncthreads();
+    if (tid == 0) {  // the next point's counts: last read before the barrier that ended point p - 1
+      s_ncav[par ^ 1] = s_nfac[par ^ 1] = 0;
+      s_dup[par ^ 1] = -1;
+    }
+    // 1. duplicates, conflict region.  A point equal to an inserted vertex is
+    // skipped and recorded, as the rounds do before any search (its conflict
+    // region need not be empty: the perturbation of an equal vertex with a
+    // larger id puts it inside)
     for (int l = tid; l < ql; l += kSeedThreads) {
-      if (!ins[l]) continue;
       const vdp::FPt& a = fp[l];
-      if (a.hx == fq.hx && a.hy == fq.hy && a.hz == fq.hz && a.lx == fq.lx && a.ly == fq.ly && a.lz == fq.lz &&
+      if (a.hx == fq.hx && a.hy == fq.hy && a.hz == fq.hz && dup[l] == 0 &&
           same_point_bits(load_pt(T, gid[l]), load_pt(T, qv)))
-        s_dupof = gid[l];
+        s_dup[par] = l;
+    }
+    auto test = [&](int s, const vdp::Sph& c) {
+      int side = vdp::sphere_side<D>(c, fq);
+      ++ntests;
+      if (side != 0) {
+        tl.f32++;
+      } else {
+        const ushort4 v = sv[s];
+        vdp::FPt fv[NV];
+        int kv[NV];
+        for (int j = 0; j < NV; ++j) {
+          const int l = get4(v, j);
+          kv[j] = gid[l];
+          fv[j] = fp[l];
+        }
+        auto load64 = [&](vdp::VPt* v64, vdp::VPt& q64) {
+          for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, kv[j]);
+          q64 = load_pt(T, qv);
+        };
+        side = vdp::in_conflict_hl<D, 1>(fv, kv, fq, qv, tl, perr, load64) ? 1 : -1;
+      }
+      if (side > 0) {
+        const int k = atomicAdd(&s_ncav[par], 1);
+        if (k < C::F) cav[k] = (unsigned short)s;
+        mark[s] = (unsigned short)(p + 1);
+      }
+    };
+    // the last star's simplices, one a thread from the block's end: the scan
+    // passes over their slots
+    const int jf = kSeedThreads - 1 - tid;
+    vdp::Sph made{};
+    int made_at = -1;
+    const int scanners = nfresh <= kSeedThreads / 2 ? kSeedThreads - ((nfresh + 31) & ~31) : kSeedThreads;
+    int sc = tid < scanners ? tid : ns;
+    bool own = jf < nfresh;
+    // one loop for both, so that the test is in the code once
+    while (own || sc < ns) {
+      int at;
+      vdp::Sph c;
+      if (own) {
+        own = false;
+        at = fresh[jf];
+        const ushort4 v = sv[at];
+        if (v.x == NONE) continue;
+        vdp::FPt lv[NV];
+        for (int i = 0; i < NV; ++i) lv[i] = fp[get4(v, i)];
+        c = made = vdp::sphere_of<D>(lv);
+        made_at = at;
+      } else {
+        at = sc;
+        sc += scanners;
+        const float4 t = sph[at];
+        if (t.w == kNoSphere) continue;
+        c = vdp::Sph{t.x, t.y, t.z, t.w};
+      }
+      test(at, c);
     }
     __syncthreads();
-    if (s_dupof >= 0) {
-      if (tid == 0) {
-        if (s_ndup >= C::DUP) s_abort = 1;
-        else dl[s_ndup++] = make_int2(qv, s_dupof);
-      }
-      __syncthreads();
-      if (s_abort) break;
+    if (s_dup[par] >= 0) {
+      if (tid == 0) dup[ql] = (unsigned short)(s_dup[par] + 1);
+      __syncthreads();  // before the next point resets this one's counts
       continue;
     }
-    // 1. conflict region: every live simplex, exact perturbed test
-    for (int s = tid; s < ns; s += kSeedThreads) {
-      const int4 v = sv[s];
-      if (v.x < 0) continue;
-      vdp::FPt fv[NV];
-      int kv[NV];
-      for (int j = 0; j < NV; ++j) {
-        const int l = get4(v, j);
-        kv[j] = gid[l];
-        fv[j] = fp[l];
-      }
-      ++ntests;
-      auto load64 = [&](vdp::VPt* v64, vdp::VPt& q64) {
-        for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, kv[j]);
-        q64 = load_pt(T, qv);
-      };
-      if (vdp::in_conflict_hl<D, 1>(fv, kv, fq, qv, tl, perr, load64)) {
-        const int k = atomicAdd(&s_ncav, 1);
-        if (k < C::C) cav[k] = s;
-        mark[s] = p + 1;
-      }
-    }
-    __syncthreads();
-    const int ncav = s_ncav;
-    if (ncav > C::C) break;  // s_abort is set below, by thread 0
-    if (ncav == 0) {
+    const int ncav = s_ncav[par];
+    if (ncav > C::F || ncav == 0) {
       // a point that is no vertex lies in the closed simplex that contains
       // it, and so inside its circumsphere: an empty region is a fault
-      if (tid == 0) {
-        set_error(T.ctr, E_INTERNAL);
-        s_abort = 1;
-      }
-      __syncthreads();
+      if (ncav == 0 && tid == 0) set_error(T.ctr, E_INTERNAL);
+      abort = true;
       break;
     }
-    // 2. boundary facets: faces of the region whose neighbour is outside it
-    // (the ridge table's halves are emptied meanwhile)
-    for (int i = tid; i < C::H; i += kSeedThreads) {
-      ha[i] = -1;
-      hb[i] = -1;
-    }
-    for (int it = tid; it < ncav * NV; it += kSeedThreads) {
-      const int k = it / NV, f = it - k * NV;
+    // 2. boundary facets: faces of the region whose neighbour is outside it;
+    // four lanes a face, one for each of the facet's faces through the new
+    // point, which takes the first or the second half of its ridge (the face's
+    // other old vertices)
+    const int gf = tid & 3;
+    for (int it0 = 0; it0 < ncav * NV; it0 += kSeedThreads / 4) {
+      const int it = it0 + (tid >> 2);
+      const bool in = it < ncav * NV;
+      const int k = in ? it / NV : 0, f = it - k * NV;
       const int s = cav[k];
-      const int code = get4(sn[s], f);
-      if (code >= 0 && mark[code >> 2] == p + 1) continue;
-      const int j = atomicAdd(&s_nfac, 1);
-      if (j < C::F) {
-        fnv[j] = set4(sv[s], f, ql);
-        fcode[j] = code;
-        fqf[j] = f;
+      const int code = get4(sn[s], in ? f : 0);
+      const bool facet = in && (code == NONE || mark[code >> 2] != p + 1);
+      const unsigned m = __ballot_sync(FULL, facet) & 0x11111111u;  // one lane of each four
+      int j = 0;
+      if ((tid & 31) == 0 && m) j = atomicAdd(&s_nfac[par], __popc(m));
+      j = __shfl_sync(FULL, j, 0) + __popc(m & ((1u << (tid & 28)) - 1u));
+      if (!facet || j >= C::F) continue;
+      const unsigned long long v = seed_replace(*reinterpret_cast<const unsigned long long*>(sv + s), f, ql);
+      if (gf == f) {
+        *reinterpret_cast<unsigned long long*>(fnv + j) = v;
+        fcode[j] = (unsigned short)code;
+        fqf[j] = (unsigned short)f;
+        continue;
       }
-    }
-    __syncthreads();
-    const int nfac = s_nfac;
-    if (nfac > C::F || ns + max(0, nfac - ncav) > C::S) break;
-    // 3a. ridge table: each face through the new point, keyed by its other
-    // old vertices (3D: two, 2D: one), takes the first or the second half
-    const unsigned long long ep = (unsigned long long)(p + 1) << 32;
-    for (int it = tid; it < nfac * NV; it += kSeedThreads) {
-      const int j = it / NV, gf = it - j * NV, qf = fqf[j];
-      if (gf == qf) continue;
-      int r[4] = {fnv[j].x, fnv[j].y, fnv[j].z, fnv[j].w};
-      int r0, r1;
-      ridge_of<D>(r, gf, qf, r0, r1);
-      const unsigned long long key = ep | ((unsigned long long)(unsigned)(r0 & 0xffff) << 16) | (unsigned)(r1 & 0xffff);
-      unsigned h = seed_hash(r0, r1, C::H);
+      if (gf >= NV) continue;
+      const unsigned key = seed_key<D>(p + 1, v, gf, f);
+      unsigned h = seed_hash(key, C::H);
       for (int probe = 0; probe < C::H; ++probe, h = (h + 1) & (unsigned)(C::H - 1)) {
-        unsigned long long cur = hk[h];
-        if ((cur >> 32) != (unsigned long long)(p + 1)) {
-          const unsigned long long old = atomicCAS(&hk[h], cur, key);
+        unsigned cur = hk[h];
+        if ((cur >> 20) != (unsigned)(p + 1)) {  // an entry of an earlier point
+          const unsigned old = atomicCAS(&hk[h], cur, key);
           if (old == cur) {
-            ha[h] = (j << 2) | gf;
+            ha[h] = (unsigned short)((j << 2) | gf);
             break;
           }
           cur = old;
         }
         if (cur == key) {
-          hb[h] = (j << 2) | gf;
+          hb[h] = (unsigned short)((j << 2) | gf);
           break;
         }
       }
     }
+    if (made_at >= 0) sph[made_at] = make_float4(made.x, made.y, made.z, made.w);
     __syncthreads();
-    // 3b. new simplices: facet j takes region slot cav[j], or a fresh slot
-    for (int j = tid; j < nfac; j += kSeedThreads) {
+    const int nfac = s_nfac[par];
+    if (nfac > C::F || ns + max(0, nfac - ncav) > C::S) {
+      abort = true;
+      break;
+    }
+    // 3. new simplices: facet j takes region slot cav[j], or a fresh slot; its
+    // outer neighbour is relinked; region slots without a facet die.  Four
+    // lanes a simplex, one for each of its links.
+    for (int j = tid >> 2; j < max(nfac, ncav); j += kSeedThreads / 4) {
       const int slot = j < ncav ? cav[j] : ns + (j - ncav);
-      const int qf = fqf[j];
-      const int4 nv = fnv[j];
-      int r[4] = {nv.x, nv.y, nv.z, nv.w};
-      int4 nn = make_int4(-1, -1, -1, -1);
-      for (int gf = 0; gf < NV; ++gf) {
-        if (gf == qf) {
-          nn = set4(nn, gf, fcode[j]);
-          continue;
+      if (j >= nfac) {
+        if (gf == 0) {
+          sv[slot].x = NONE;
+          sph[slot].w = kNoSphere;
         }
-        int r0, r1;
-        ridge_of<D>(r, gf, qf, r0, r1);
-        const unsigned long long key = ep | ((unsigned long long)(unsigned)(r0 & 0xffff) << 16) | (unsigned)(r1 & 0xffff);
-        const int h = seed_find(hk, C::H, key, r0, r1);
+        continue;
+      }
+      const int qf = fqf[j], code = fcode[j];
+      const unsigned long long v = *reinterpret_cast<const unsigned long long*>(fnv + j);
+      unsigned short link = NONE;
+      if (gf == qf) {
+        link = (unsigned short)code;
+        *reinterpret_cast<unsigned long long*>(sv + slot) = v;
+        sph[slot].w = kNoSphere;  // in `fresh`: see step 1
+        fresh[j] = (unsigned short)slot;
+        if (code != NONE)
+          reinterpret_cast<unsigned short*>(sn + (code >> 2))[code & 3] = (unsigned short)((slot << 2) | qf);
+      } else if (gf < NV) {
+        const unsigned key = seed_key<D>(p + 1, v, gf, qf);
+        unsigned h = seed_hash(key, C::H);
+        for (int probe = 0; probe < C::H && hk[h] != key && (hk[h] >> 20) == (unsigned)(p + 1); ++probe)
+          h = (h + 1) & (unsigned)(C::H - 1);
         const int mine = (j << 2) | gf;
-        const int other = h < 0 ? -1 : (ha[h] == mine ? hb[h] : ha[h]);
-        if (other < 0 || (other >> 2) >= nfac) {
+        const int other = hk[h] != key ? mine : (ha[h] == mine ? hb[h] : ha[h]);
+        if (other == mine || (other >> 2) >= nfac) {
           set_error(T.ctr, E_INTERNAL);  // a ridge with one half: not a closed star
           s_abort = 1;
           continue;
         }
         const int oj = other >> 2;
         const int oslot = oj < ncav ? cav[oj] : ns + (oj - ncav);
-        nn = set4(nn, gf, (oslot << 2) | (other & 3));
+        link = (unsigned short)((oslot << 2) | (other & 3));
       }
-      sv[slot] = nv;
-      sn[slot] = nn;
+      reinterpret_cast<unsigned short*>(sn + slot)[gf] = link;
     }
-    __syncthreads();
-    // 3c. outer neighbours point at the new simplices; region slots without a
-    // facet die (their records are not read again)
-    for (int j = tid; j < nfac; j += kSeedThreads) {
-      const int code = fcode[j];
-      if (code < 0) continue;
-      const int slot = j < ncav ? cav[j] : ns + (j - ncav);
-      reinterpret_cast<int*>(sn + (code >> 2))[code & 3] = (slot << 2) | fqf[j];
-    }
-    for (int k = nfac + tid; k < ncav; k += kSeedThreads) sv[cav[k]].x = -1;
-    __syncthreads();
-    if (tid == 0) {
-      s_ns = ns + max(0, nfac - ncav);
-      s_ncav = 0;
-      s_nfac = 0;
-      s_nins += 1;
-      s_created += nfac;
-      s_killed += ncav;
-      s_maxc = max(s_maxc, ncav);
-      s_maxf = max(s_maxf, nfac);
-      s_holes += max(0, ncav - nfac);
-      ins[ql] = 1;
-    }
+    ns += max(0, nfac - ncav);
+    nfresh = nfac;
+    nins += 1;
+    ncreated += nfac;
+    nkilled += ncav;
+    maxc = max(maxc, ncav);
+    maxf = max(maxf, nfac);
+    holes += max(0, ncav - nfac);
     __syncthreads();
     if (s_abort) break;
   }
-  // a loop left early (capacity) has not finished its point
-  if (tid == 0 && (s_ncav > C::C || s_nfac > C::F || s_ncav != 0 || s_nfac != 0)) s_abort = 1;
   __syncthreads();
   if (perr) set_error(T.ctr, E_PRECISION);
-  if (s_abort) return;  // nothing written: the rounds insert these points
+  if (abort || s_abort) return;  // nothing written: the rounds insert these points
   // write-out: live slots are ranked (mark[] holds the ranks) and stored
   // compacted with global vertex ids and neighbour codes
-  const int ns = s_ns;
   __shared__ int wsum[kSeedThreads / 32];
   constexpr int PER = (C::S + kSeedThreads - 1) / kSeedThreads;
   int cnt = 0;
   for (int k = 0; k < PER; ++k) {
     const int s = tid * PER + k;
-    cnt += (s < ns && sv[s].x >= 0) ? 1 : 0;
+    cnt += (s < ns && sv[s].x != NONE) ? 1 : 0;
   }
   int incl = cnt;
   for (int o = 1; o < 32; o <<= 1) {
@@ -2679,7 +2729,7 @@ __global__ void __launch_bounds__(kSeedThreads, 1) k_seed(DevTree T, int npts, i
   base += incl - cnt;
   for (int k = 0; k < PER; ++k) {
     const int s = tid * PER + k;
-    if (s < ns && sv[s].x >= 0) mark[s] = base++;
+    if (s < ns && sv[s].x != NONE) mark[s] = (unsigned short)base++;
   }
   __syncthreads();
   int nlive = 0;
@@ -2689,41 +2739,49 @@ __global__ void __launch_bounds__(kSeedThreads, 1) k_seed(DevTree T, int npts, i
     return;
   }
   for (int s = tid; s < ns; s += kSeedThreads) {
-    const int4 v = sv[s];
-    if (v.x < 0) continue;
-    const int4 n = sn[s];
+    const ushort4 v = sv[s];
+    if (v.x == NONE) continue;
+    const ushort4 n = sn[s];
+    const int slot = mark[s];  // < nlive <= cap_simp
     int4 gv = make_int4(-1, -1, -1, -1), gn = make_int4(-1, -1, -1, -1);
+    vdp::FPt lv[NV];
     for (int j = 0; j < NV; ++j) {
-      gv = set4(gv, j, gid[get4(v, j)]);
-      const int c = get4(n, j);
-      gn = set4(gn, j, c < 0 ? -1 : (mark[c >> 2] << 2) | (c & 3));
+      const int l = get4(v, j), c = get4(n, j);
+      gv = set4(gv, j, gid[l]);
+      gn = set4(gn, j, c == NONE ? -1 : (mark[c >> 2] << 2) | (c & 3));
+      home[l] = (unsigned short)slot;
+      lv[j] = fp[l];
     }
-    store_simplex(T, mark[s], gv, gn);
+    store_simplex(T, slot, gv, gn);
     if (D == 3) {
-      vdp::FPt lv[NV];
-      for (int j = 0; j < NV; ++j) lv[j] = fp[get4(v, j)];
       const vdp::Sph c = vdp::sphere_of<D>(lv);
-      *reinterpret_cast<float4*>(T.sph + mark[s]) = make_float4(c.x, c.y, c.z, c.w);  // mark[s] < nlive <= cap_simp
+      *reinterpret_cast<float4*>(T.sph + slot) = make_float4(c.x, c.y, c.z, c.w);
     }
-    for (int j = 0; j < NV; ++j) {
-      const int l = get4(v, j);
-      if (l >= NV) write_hints<D>(T, gid[l], fp[l], mark[s]);
+  }
+  __syncthreads();
+  // one hint per point (each of its simplices is a valid walk start), the
+  // duplicates
+  const int d0 = T.ctr->ndup;
+  for (int l = NV + tid; l < NV + npts; l += kSeedThreads) {
+    if (dup[l] == 0) {
+      write_hints<D>(T, gid[l], fp[l], home[l]);
+    } else {
+      const int k = d0 + atomicAdd(&s_ndup, 1);
+      if (k < T.cap_dups) T.dups[k] = make_int2(gid[l], gid[dup[l] - 1]);
     }
   }
   flush_tally(T.ctr, tl, ntests, 0);
+  __syncthreads();
   if (tid == 0) {
     Counters* c = T.ctr;
     c->nsimp = nlive;
-    c->ninserted += s_nins;
-    c->winners += s_nins;
-    c->created += s_created;
-    c->killed += s_killed;
-    c->holes += s_holes;
-    c->max_cav = max(c->max_cav, s_maxc);
-    c->max_fac = max(c->max_fac, s_maxf);
-    const int d0 = c->ndup;
-    for (int k = 0; k < s_ndup; ++k)
-      if (d0 + k < T.cap_dups) T.dups[d0 + k] = dl[k];
+    c->ninserted += nins;
+    c->winners += nins;
+    c->created += ncreated;
+    c->killed += nkilled;
+    c->holes += holes;
+    c->max_cav = max(c->max_cav, maxc);
+    c->max_fac = max(c->max_fac, maxf);
     c->ndup = d0 + s_ndup;
     c->lev_next = nlev;
   }

@@ -1068,6 +1068,23 @@ VDP_HD uint32_t f32_bits(float f) {
 #endif
 }
 
+// 0.5 / x and 1 / sqrt(x) to a few units in the last place: the centre may be
+// any point near the true one, and the bounds below have room for it.
+VDP_HD float half_over(float x) {
+#if defined(__CUDA_ARCH__)
+  return __fdividef(0.5f, x);
+#else
+  return 0.5f / x;
+#endif
+}
+VDP_HD float inv_sqrt(float x) {
+#if defined(__CUDA_ARCH__)
+  return rsqrtf(x);
+#else
+  return 1.0f / sqrtf(x);
+#endif
+}
+
 // Squared distance of p to the stored centre (see above); NaN if p's split is
 // not accurate.
 template <int D>
@@ -1098,7 +1115,7 @@ VDP_HD Sph sphere_of(const FPt* v) {
   L += flag;
   if (!(L >= 2.98023223876953125e-8f && L <= 1048576.0f && M <= 1048576.0f * L)) return out;
   // n[i]: 1-norm of the cofactor row that goes with d_i
-  float det, n[D], ox, oy, oz = 0.0f, floor_det;
+  float det, n[D], ox, oy, oz = 0.0f, floor_det, hd;
   const float L2 = L * L;
   if (D == 3) {
     const float px = ffma(y[1], z[2 % D], -(z[1] * y[2 % D])), py = ffma(z[1], x[2 % D], -(x[1] * z[2 % D])),
@@ -1111,7 +1128,8 @@ VDP_HD Sph sphere_of(const FPt* v) {
     const float a2 = ffma(z[0], z[0], ffma(y[0], y[0], x[0] * x[0]));
     const float b2 = ffma(z[1], z[1], ffma(y[1], y[1], x[1] * x[1]));
     const float c2 = ffma(z[2 % D], z[2 % D], ffma(y[2 % D], y[2 % D], x[2 % D] * x[2 % D]));
-    const float h = 0.5f / det;
+    hd = half_over(det);
+    const float h = hd;
     ox = (a2 * px + b2 * qx + c2 * rx) * h;
     oy = (a2 * py + b2 * qy + c2 * ry) * h;
     oz = (a2 * pz + b2 * qz + c2 * rz) * h;
@@ -1122,7 +1140,8 @@ VDP_HD Sph sphere_of(const FPt* v) {
   } else {
     det = ffma(x[0], y[1], -(y[0] * x[1]));
     const float a2 = ffma(y[0], y[0], x[0] * x[0]), b2 = ffma(y[1], y[1], x[1] * x[1]);
-    const float h = 0.5f / det;
+    hd = half_over(det);
+    const float h = hd;
     ox = (a2 * y[1] - b2 * y[0]) * h;
     oy = (b2 * x[0] - a2 * x[1]) * h;
     n[0] = fabsf(x[1]) + fabsf(y[1]);
@@ -1142,8 +1161,8 @@ VDP_HD Sph sphere_of(const FPt* v) {
   const float nslack = D == 3 ? 1.52587890625e-5f * L2 : 1.52587890625e-5f * L;  // 2^-16
   float e = 0.0f;
   for (int i = 0; i < D; ++i) e += (fabsf(r[i] - r0) + slack) * (n[i] + nslack);
-  e = 0.6f * e / fabsf(det);  // 1 / (2 * 7/8) and the rounding of this sum
-  const float width = 4.6f * e / sqrtf(r0) + 4.2e-6f;  // 4.25 E / r_0 + 20u + 2^-19, rounded up
+  e *= 1.2f * fabsf(hd);  // 1 / (2 |det| 7/8), and the rounding of this sum and of hd
+  const float width = 4.6f * e * inv_sqrt(r0) + 4.2e-6f;  // 4.25 E / r_0 + 20u + 2^-19, rounded up
   const float cm = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz)));
   if (!(width < 0.25f && r0 <= 1.2089258196146292e24f && cm * cm <= 4.398046511104e12f * r0)) return out;
   // width < 2^(ex + 1) with ex the exponent of width: bits = -3 - ex, at most 15
