@@ -141,8 +141,16 @@ struct vd_tree {
   int* h_pair = nullptr;
   unsigned long long* d_check = nullptr;
   int* d_misc = nullptr;      // small device scratch (live-slot search, locate)
-  int64_t* d_loc = nullptr;
-  int64_t cap_loc = 0;
+  // buffers of vd_locate_points, kept from call to call and sized by the largest
+  struct LocateScratch {
+    int *flags = nullptr, *rank = nullptr, *tmp = nullptr;  // per slot
+    int64_t cap_slots = 0;
+    double* q = nullptr;  // per query of a chunk
+    int2* res = nullptr;
+    int64_t cap_q = 0;
+    int* out = nullptr;  // ranks of a chunk's regions
+    int64_t cap_out = 0;
+  } loc;
   int64_t ncells = 0;
   // pinned staging for small host<->device copies
   unsigned long long* h_mm = nullptr;
@@ -437,7 +445,12 @@ void release(vd_tree* t) {
   dfree(t->d_pair);
   dfree(t->d_check);
   dfree(t->d_misc);
-  dfree(t->d_loc);
+  dfree(t->loc.flags);
+  dfree(t->loc.rank);
+  dfree(t->loc.tmp);
+  dfree(t->loc.q);
+  dfree(t->loc.res);
+  dfree(t->loc.out);
   dfree(t->d_counts);
   dfree(t->T.lev_off);
   dfree(t->T.hint);
@@ -1795,6 +1808,56 @@ int vd_autotune_batch(vd_tree* t, const double* d_pts, const int64_t* offsets, i
   return rc;
 }
 
+// The m queries of S.q (numbers q0 ..) of vd_locate_points by the thread form,
+// whose per-query room grows with the largest region.
+static int locate_large(vd_tree* t, const vd::Launch& L, int nsimp, int64_t q0, int m, int64_t* offsets, int64_t* ids,
+                        int64_t cap, int64_t& total, bool& outside) {
+  const int dim = t->dim;
+  vd_tree::LocateScratch& S = t->loc;
+  int *rank = nullptr, *flags = nullptr, *tmp = nullptr, *out = nullptr, *cnt = nullptr;
+  int cap_per = 256, rc = vd::E_OK;
+  std::vector<int> hc(m), ho;
+  if (dalloc(&flags, nsimp + 1) || dalloc(&rank, nsimp + 1) || dalloc(&tmp, vd::scan_scratch_ints(nsimp + 1)) ||
+      dalloc(&cnt, m) || dalloc(&out, (size_t)m * cap_per))
+    rc = vd::E_NOMEM;
+  if (!rc) vd::launch_live_rank(t->T, L, nsimp, flags, rank, tmp);
+  while (!rc) {
+    vd::launch_locate(t->T, L, dim, S.q, m, cap_per, rank, out, cnt);
+    cudaMemcpyAsync(hc.data(), cnt, sizeof(int) * m, cudaMemcpyDeviceToHost, t->stream);
+    rc = cuda_status(cudaStreamSynchronize(t->stream));
+    int need = 0;
+    for (int i = 0; i < m; ++i) need = std::max(need, hc[i]);
+    if (rc || need <= cap_per) break;
+    // a region larger than the per-query room (what did not fit was not
+    // searched on, so its true size is not known): once more with more
+    cap_per = std::max(need, 2 * cap_per);
+    dfree(out);
+    if (dalloc(&out, (size_t)m * cap_per)) rc = vd::E_NOMEM;
+  }
+  if (!rc) {
+    ho.resize((size_t)m * cap_per);
+    cudaMemcpyAsync(ho.data(), out, sizeof(int) * ho.size(), cudaMemcpyDeviceToHost, t->stream);
+    rc = cuda_status(cudaStreamSynchronize(t->stream));
+  }
+  for (int i = 0; i < m && !rc; ++i) {
+    const int c = std::max(hc[i], 0);
+    outside = outside || hc[i] < 0;
+    offsets[q0 + i + 1] = offsets[q0 + i] + c;
+    if (ids && total + c <= cap) {
+      int64_t* dst = ids + total;
+      for (int k = 0; k < c; ++k) dst[k] = ho[(size_t)i * cap_per + k];
+      std::sort(dst, dst + c);
+    }
+    total += c;
+  }
+  dfree(flags);
+  dfree(rank);
+  dfree(tmp);
+  dfree(cnt);
+  dfree(out);
+  return rc;
+}
+
 int vd_locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets, int64_t* ids, int64_t cap) {
   if (ready(t) || !t->has_geometry || t->nsets != 1 || nq < 0 || (nq > 0 && !pts) || !offsets) return VD_ERR_ARG;
   offsets[0] = 0;
@@ -1804,63 +1867,68 @@ int vd_locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets
   const int dim = t->dim;
   const int nsimp = t->hctr->nsimp;
   const vd::Launch L = launch_of(t);
-  int *flags = nullptr, *rank = nullptr, *tmp = nullptr, *out = nullptr, *cnt = nullptr;
-  double* dq = nullptr;
   const int64_t chunk = std::min<int64_t>(nq, 1 << 16);
-  int cap_per = 256;
-  if (dalloc(&flags, nsimp + 1) || dalloc(&rank, nsimp + 1) || dalloc(&tmp, vd::scan_scratch_ints(nsimp + 1)) ||
-      dalloc(&dq, (size_t)(chunk * dim)) || dalloc(&cnt, chunk) || dalloc(&out, (size_t)(chunk * cap_per))) {
-    rc = vd::E_NOMEM;
+  vd_tree::LocateScratch& S = t->loc;
+  // ranks are needed for ids only, and the counts-only call makes none
+  if (ids && nsimp + 1 > S.cap_slots) {
+    dfree(S.flags);
+    dfree(S.rank);
+    dfree(S.tmp);
+    S.cap_slots = 0;
+    const int64_t c = nsimp + 1 + nsimp / 8;
+    if (dalloc(&S.flags, c) || dalloc(&S.rank, c) || dalloc(&S.tmp, vd::scan_scratch_ints(c))) return VD_ERR_NOMEM;
+    S.cap_slots = c;
   }
-  if (!rc) vd::launch_live_rank(t->T, L, nsimp, flags, rank, tmp);
-  std::vector<int> hc(chunk), ho;
+  if (chunk > S.cap_q) {
+    dfree(S.q);
+    dfree(S.res);
+    S.cap_q = 0;
+    if (dalloc(&S.q, (size_t)(chunk * dim)) || dalloc(&S.res, chunk + 1)) return VD_ERR_NOMEM;
+    S.cap_q = chunk;
+  }
+  if (ids) vd::launch_live_rank(t->T, L, nsimp, S.flags, S.rank, S.tmp);
+  std::vector<int2> hr(chunk + 1);
+  std::vector<int> ho;
   bool outside = false;
   int64_t total = 0;
   for (int64_t q0 = 0; q0 < nq && !rc; q0 += chunk) {
     const int m = (int)std::min<int64_t>(chunk, nq - q0);
-    cudaMemcpyAsync(dq, pts + q0 * dim, sizeof(double) * m * dim, cudaMemcpyHostToDevice, t->stream);
-    vd::launch_locate(t->T, L, dim, dq, m, cap_per, rank, out, cnt);
-    cudaMemcpyAsync(hc.data(), cnt, sizeof(int) * m, cudaMemcpyDeviceToHost, t->stream);
-    if (cudaStreamSynchronize(t->stream) != cudaSuccess) {
-      rc = vd::E_CUDA;
-      break;
-    }
-    int need = 0;
-    for (int i = 0; i < m; ++i) need = std::max(need, hc[i]);
-    if (need > cap_per) {  // a region larger than the per-query room: rerun this chunk with enough
-      cap_per = need;
-      dfree(out);
-      if (dalloc(&out, (size_t)m * cap_per)) {
-        rc = vd::E_NOMEM;
-        break;
+    cudaMemcpyAsync(S.q, pts + q0 * dim, sizeof(double) * m * dim, cudaMemcpyHostToDevice, t->stream);
+    int64_t want = ids ? std::max<int64_t>(S.cap_out, (dim == 3 ? 40LL : 12LL) * m + 256) : 0;
+    bool large = false;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+      if (want > S.cap_out) {
+        dfree(S.out);
+        S.cap_out = 0;
+        if (want > 0x7fffffffLL || dalloc(&S.out, (size_t)want)) return VD_ERR_NOMEM;
+        S.cap_out = want;
       }
-      vd::launch_locate(t->T, L, dim, dq, m, cap_per, rank, out, cnt);
-      cudaMemcpyAsync(hc.data(), cnt, sizeof(int) * m, cudaMemcpyDeviceToHost, t->stream);
+      vd::launch_locate_warp(t->T, L, dim, S.q, m, S.rank, ids ? S.out : nullptr, (int)S.cap_out, S.res);
+      cudaMemcpyAsync(hr.data(), S.res, sizeof(int2) * (m + 1), cudaMemcpyDeviceToHost, t->stream);
+      if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
+      if (!ids || hr[m].x <= S.cap_out) break;
+      want = hr[m].x;  // more ranks than the first guess: once more with enough room
     }
-    ho.resize((size_t)m * cap_per);
-    cudaMemcpyAsync(ho.data(), out, sizeof(int) * ho.size(), cudaMemcpyDeviceToHost, t->stream);
-    if (cudaStreamSynchronize(t->stream) != cudaSuccess) {
-      rc = vd::E_CUDA;
-      break;
+    for (int i = 0; i < m; ++i) large = large || hr[i].x == -2;
+    if (large) {
+      rc = locate_large(t, L, nsimp, q0, m, offsets, ids, cap, total, outside);
+      continue;
+    }
+    const int k = hr[m].x;
+    if (ids && k > 0) {
+      ho.resize(k);
+      cudaMemcpyAsync(ho.data(), S.out, sizeof(int) * k, cudaMemcpyDeviceToHost, t->stream);
+      if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
     }
     for (int i = 0; i < m; ++i) {
-      const int c = std::max(hc[i], 0);
-      outside = outside || hc[i] < 0;
+      const int c = std::max(hr[i].x, 0);
+      outside = outside || hr[i].x < 0;
       offsets[q0 + i + 1] = offsets[q0 + i] + c;
-      if (ids && total + c <= cap) {
-        int64_t* dst = ids + total;
-        for (int k = 0; k < c; ++k) dst[k] = ho[(size_t)i * cap_per + k];
-        std::sort(dst, dst + c);
-      }
+      if (ids && total + c <= cap) std::copy(ho.begin() + hr[i].y, ho.begin() + hr[i].y + c, ids + total);
       total += c;
     }
   }
-  dfree(flags);
-  dfree(rank);
-  dfree(tmp);
-  dfree(dq);
-  dfree(cnt);
-  dfree(out);
+  if (!rc) rc = sync_counters(t);
   if (rc) return rc;
   if (t->hctr->err) return t->hctr->err;
   if (ids && total > cap) return VD_ERR_ARG;

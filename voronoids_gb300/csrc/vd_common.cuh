@@ -351,6 +351,12 @@ void scan_ints(const int* in, int* out, int64_t n, int* tmp, cudaStream_t st);
 void launch_locate(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, int cap_per,
                    const int* rank, int* out, int* counts);
 void launch_live_rank(const DevTree& T, const Launch& L, int nsimp, int* flags, int* rank, int* tmp);
+// The same, a warp per query: res[i] = (count, first) with the sorted ranks of
+// query i at out[first ..], count -1 outside the super simplex, -2 too large
+// for a warp (launch_locate does it); res[nq].x = ranks in all, which may
+// exceed cap_out.  out null: counts only.
+void launch_locate_warp(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, const int* rank, int* out,
+                        int cap_out, int2* res);
 // Circumcentre (3 doubles, z = 0 in 2D) and radius of each live simplex,
 // written at its rank.
 void launch_circum(const DevTree& T, const Launch& L, int dim, int nsimp, const int* rank, double* centers,

@@ -156,14 +156,18 @@ class DelaunayTree:
         off = np.zeros(nq + 1, dtype=np.int64)
         L = _native.load()
         i64p = ctypes.POINTER(ctypes.c_int64)
-        rc = L.vd_locate_points(self._h, _dp(q), nq, off.ctypes.data_as(i64p), None, 0)
+        cap = (48 if self.dim == 3 else 16) * nq + 256  # above the usual region sizes
+        for _ in range(2):
+            ids = np.empty(cap, dtype=np.int64)
+            rc = L.vd_locate_points(self._h, _dp(q), nq, off.ctypes.data_as(i64p), ids.ctypes.data_as(i64p), cap)
+            if rc == 1 and int(off[-1]) > cap:  # more ids than the first guess: exact size
+                cap = int(off[-1])
+                continue
+            break
         if rc not in (_native.VD_OK, 6):
             _check(rc, "locate")
-        ids = np.zeros(max(int(off[-1]), 1), dtype=np.int64)
-        rc = L.vd_locate_points(self._h, _dp(q), nq, off.ctypes.data_as(i64p), ids.ctypes.data_as(i64p), ids.shape[0])
-        if rc not in (_native.VD_OK, 6):
-            _check(rc, "locate")
-        out = [ids[off[i]:off[i + 1]] for i in range(nq)]
+        o = off.tolist()
+        out = [ids[a:b] for a, b in zip(o, o[1:])]
         return out[0] if single else out
 
     def num_sets(self):
