@@ -180,7 +180,8 @@ struct vd_tree {
     uint64_t seed;
     float ratio;
     long long launches;
-    cudaGraphExec_t exec;
+    int64_t call;          // the call that first asked for it
+    cudaGraphExec_t exec;  // null: asked for, not captured
   };
   std::vector<ChunkGraph> graphs;
   bool use_graphs = true;
@@ -394,7 +395,8 @@ int ensure_points(vd_tree* t, int64_t n_new) {
 }
 
 void drop_graphs(vd_tree* t) {
-  for (auto& g : t->graphs) cudaGraphExecDestroy(g.exec);
+  for (auto& g : t->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   t->graphs.clear();
 }
 
@@ -739,12 +741,10 @@ vd::Launch sized_launch(const vd_tree* t, int64_t items) {
   return L;
 }
 
-// Launches `chunk` rounds as one CUDA graph, capturing it on first use.
-// Returns false (nothing launched) when graphs are off for this tree:
-// profiling and tracing need per-kernel events, and a failed capture turns
-// graphs off.
-bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Feed& fd) {
-  if (!t->use_graphs || t->prof || t->trace) return false;
+// The graph of `chunk` rounds for these launches, or null when there is none
+// yet.  A chunk of several rounds that an earlier call has asked for is captured;
+// asked for the first time it is only noted.
+vd_tree::ChunkGraph* chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Feed& fd) {
   vd_tree::ChunkGraph* hit = nullptr;
   for (auto& g : t->graphs)
     if (g.chunk == chunk && g.blocks == L.blocks && g.warps == L.warps && g.passes == t->tuning.passes &&
@@ -756,24 +756,7 @@ bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Fe
       break;
     }
   if (!hit) {
-    if (t->graphs.size() >= 24) drop_graphs(t);
-    const long long before = vd::launches_total();
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    bool ok = cudaStreamBeginCapture(t->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    if (ok) {
-      for (int k = 0; k < chunk; ++k) vd::launch_round(t->T, L, t->dim, t->tuning, fd, nullptr);
-      ok = cudaStreamEndCapture(t->stream, &graph) == cudaSuccess && graph;
-    }
-    if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-    if (graph) cudaGraphDestroy(graph);
-    const long long launches = vd::launches_total() - before;
-    vd::note_launches(-launches);  // counted when replayed
-    if (!ok) {
-      cudaGetLastError();
-      t->use_graphs = false;
-      return false;
-    }
+    if (t->graphs.size() >= 48) drop_graphs(t);
     vd_tree::ChunkGraph g;
     memcpy(&g.T, &t->T, sizeof(vd::DevTree));
     g.chunk = chunk;
@@ -786,17 +769,63 @@ bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Fe
     g.big_block = t->tuning.big_block;
     g.seed = fd.seed;
     g.ratio = fd.ratio;
-    g.launches = launches;
-    g.exec = exec;
+    g.launches = 0;
+    g.call = t->calls;
+    g.exec = nullptr;
     t->graphs.push_back(g);
     hit = &t->graphs.back();
   }
-  if (cudaGraphLaunch(hit->exec, t->stream) != cudaSuccess) {
+  if (hit->exec) return hit;
+  if (chunk > 1 && hit->call == t->calls) return nullptr;
+  const long long before = vd::launches_total();
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  bool ok = cudaStreamBeginCapture(t->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  if (ok) {
+    for (int k = 0; k < chunk; ++k) vd::launch_round(t->T, L, t->dim, t->tuning, fd, nullptr);
+    ok = cudaStreamEndCapture(t->stream, &graph) == cudaSuccess && graph;
+  }
+  if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  const long long launches = vd::launches_total() - before;
+  vd::note_launches(-launches);  // counted when replayed
+  if (!ok) {
     cudaGetLastError();
     t->use_graphs = false;
-    return false;
+    return nullptr;
   }
-  vd::note_launches(hit->launches);
+  hit->launches = launches;
+  hit->exec = exec;
+  return hit;
+}
+
+// Launches `chunk` rounds as a CUDA graph: one of the whole chunk once an
+// earlier call has run such a chunk, until then a graph of one round replayed
+// `chunk` times.  Capturing 8 rounds costs about 0.3 ms and saves 20 us a
+// replay, so it does not pay within one call (one-shot 10,000 points 2D: 4.6 ms
+// of insertion with chunk graphs captured at once, 4.1 with one-round graphs,
+// repeated calls 3.1 and 3.3).  Returns false (nothing launched) when graphs are
+// off for this tree: profiling and tracing need per-kernel events, and a failed
+// capture turns graphs off.
+bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Feed& fd) {
+  if (!t->use_graphs || t->prof || t->trace) return false;
+  const vd_tree::ChunkGraph* g = chunk_graph(t, L, chunk, fd);
+  int replays = 1;
+  if (!g && t->use_graphs) {
+    g = chunk_graph(t, L, 1, fd);
+    replays = chunk;
+  }
+  if (!g) return false;
+  for (int k = 0; k < replays; ++k) {
+    if (cudaGraphLaunch(g->exec, t->stream) != cudaSuccess) {
+      cudaGetLastError();
+      t->use_graphs = false;
+      if (k == 0) return false;
+      for (; k < replays; ++k) vd::launch_round(t->T, L, t->dim, t->tuning, fd, nullptr);
+      return true;
+    }
+    vd::note_launches(g->launches);
+  }
   return true;
 }
 
