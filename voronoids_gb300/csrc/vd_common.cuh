@@ -235,6 +235,16 @@ __device__ inline int set_index(const DevTree& T, int vid) {
 }
 #endif
 
+// Memory (vd_memory.cu).  Device memory in stream order from a pool of the
+// library's own on the current device; null when there is none.  pool_free
+// takes null, and a stream that is gone.
+void* pool_alloc(size_t bytes, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
+// Pinned host blocks of kPinnedBytes.
+constexpr size_t kPinnedBytes = 8192;
+void* pinned_alloc();
+void pinned_free(void* p);
+
 // Kernels launched by this library in this process (diagnostics).
 void note_launches(long long k);
 long long launches_total();
