@@ -84,6 +84,14 @@ struct Cap<2> {
   static constexpr int MAXC = 64, MAXF = 96, HS = 128;
 };
 
+// First statement of every round kernel: with Launch::early the next kernel of
+// the stream may be put on the device now (it waits here for this one to
+// finish), and this one waits for the kernel before it.
+__device__ __forceinline__ void round_kernel_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ int get4(const int4& a, int i) {
   return i == 0 ? a.x : (i == 1 ? a.y : (i == 2 ? a.z : a.w));
 }
@@ -455,7 +463,10 @@ __device__ __forceinline__ void plan_body(DevTree T, float ratio, int bid, int n
   c->feed_hi = T.lev_off[lev];
   c->lev_next = lev;
 }
-__global__ void k_plan(DevTree T, float ratio) { plan_body(T, ratio, blockIdx.x, gridDim.x); }
+__global__ void k_plan(DevTree T, float ratio) {
+  round_kernel_begin();
+  plan_body(T, ratio, blockIdx.x, gridDim.x);
+}
 
 // Activates the points planned for this round: each walks from the finest
 // available grid hint to the simplex that contains it (visibility walk,
@@ -535,7 +546,10 @@ __device__ __forceinline__ void activate_body(DevTree T, unsigned long long seed
   flush_tally(T.ctr, tl, 0, walk);
 }
 template <int D>
-__global__ void VD_WALK_BOUNDS k_activate(DevTree T, unsigned long long seed) { activate_body<D>(T, seed, blockIdx.x, gridDim.x); }
+__global__ void VD_WALK_BOUNDS k_activate(DevTree T, unsigned long long seed) {
+  round_kernel_begin();
+  activate_body<D>(T, seed, blockIdx.x, gridDim.x);
+}
 
 // ---------------------------------------------------------------------------
 template <int D>
@@ -597,7 +611,10 @@ __device__ __forceinline__ void pick_body(DevTree T, int thin, int bid, int nblk
   }
 }
 template <int D>
-__global__ void k_pick(DevTree T, int thin) { pick_body<D>(T, thin, blockIdx.x, gridDim.x); }
+__global__ void k_pick(DevTree T, int thin) {
+  round_kernel_begin();
+  pick_body<D>(T, thin, blockIdx.x, gridDim.x);
+}
 
 // Headers of a warp's items in a grid-stride loop over a candidate list,
 // staged in shared memory: lane k loads item it0 + k * nw (its candidate,
@@ -1067,7 +1084,10 @@ __device__ __forceinline__ void thin_body(DevTree T, int thin, int bid, int nblk
   }
 }
 template <int D>
-__global__ void k_thin(DevTree T, int thin) { thin_body<D>(T, thin, blockIdx.x, gridDim.x); }
+__global__ void k_thin(DevTree T, int thin) {
+  round_kernel_begin();
+  thin_body<D>(T, thin, blockIdx.x, gridDim.x);
+}
 
 template <int D>
 struct alignas(16) WarpCav {
@@ -1276,6 +1296,7 @@ __device__ __forceinline__ void cavity_body(DevTree T, int adjacent, int bid, in
 template <int D, int XT>
 __global__ void __launch_bounds__(128, VD_CAVITY_MIN_BLOCKS) k_cavity(DevTree T, int adjacent, int defer_big) {
   __shared__ WarpCav<D> smem[4];
+  round_kernel_begin();
   cavity_body<D, XT>(T, adjacent, blockIdx.x, gridDim.x, smem, defer_big != 0);
 }
 
@@ -1285,6 +1306,7 @@ template <int D, int XT>
 __global__ void __launch_bounds__(512, 1) k_cavity_big(DevTree T, int adjacent) {
   __shared__ WarpCtl ctl;
   extern __shared__ int bsm[];  // kBigSmem bytes: the search's id set, then its ready marks
+  round_kernel_begin();
   const int n = T.ctr->nbig;
   if (n == 0) return;
   const unsigned long long pe = pass_epoch(T.ctr->round, 0);
@@ -1848,6 +1870,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
 template <int D, int MODE, int XT>
 __global__ void VD_CHECK_BOUNDS k_check(DevTree T, int pass, int last, unsigned long long seed, int defer_big) {
   extern __shared__ __align__(16) unsigned char dsm[];
+  round_kernel_begin();
   check_body<D, MODE, XT>(T, pass, last, seed, blockIdx.x, gridDim.x, dsm, defer_big != 0);
 }
 
@@ -1855,6 +1878,7 @@ __global__ void VD_CHECK_BOUNDS k_check(DevTree T, int pass, int last, unsigned 
 // star, publishes its shared facets and its hints.
 template <int D>
 __global__ void __launch_bounds__(512, 1) k_commit_big(DevTree T) {
+  round_kernel_begin();
   const int n = T.ctr->nbigw;
   if (n == 0) return;
   const int round = T.ctr->round;
@@ -2002,7 +2026,10 @@ __device__ __forceinline__ void reclaim_body(DevTree T, int pass, int adjacent, 
   }
 }
 template <int D>
-__global__ void __launch_bounds__(128, 6) k_reclaim(DevTree T, int pass, int adjacent) { reclaim_body<D>(T, pass, adjacent, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(128, 6) k_reclaim(DevTree T, int pass, int adjacent) {
+  round_kernel_begin();
+  reclaim_body<D>(T, pass, adjacent, blockIdx.x, gridDim.x);
+}
 
 template <int D>
 __device__ __forceinline__ void relocate_body(DevTree T, int bid, int nblk) {
@@ -2086,7 +2113,10 @@ __device__ __forceinline__ void relocate_body(DevTree T, int bid, int nblk) {
   flush_tally(T.ctr, tl, 0, walk);
 }
 template <int D>
-__global__ void VD_WALK_BOUNDS k_relocate(DevTree T) { relocate_body<D>(T, blockIdx.x, gridDim.x); }
+__global__ void VD_WALK_BOUNDS k_relocate(DevTree T) {
+  round_kernel_begin();
+  relocate_body<D>(T, blockIdx.x, gridDim.x);
+}
 
 // ---------------------------------------------------------------------------
 // Small rounds in one launch.  While few points are active a round is a
@@ -2819,31 +2849,44 @@ void round_impl(const DevTree& T, const Launch& L, const Tuning& tu, const Feed&
     }
   };
   if (pf && pf->n == 0) cudaEventRecord(pf->ev[0], L.stream);
+  auto go = [&](auto kernel, int grid, int block, size_t smem, auto... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = L.stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = L.early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+  };
   note_launches((tu.adjacent ? 6 + 3 * tu.passes - 1 : 6 + 2 * tu.passes - 1) - (tu.thin > 0 ? 0 : 1) +
                 (tu.big_block ? 1 + (tu.adjacent ? tu.passes : 0) : 0));
-  k_plan<<<1, 32, 0, L.stream>>>(T, fd.ratio);
-  k_activate<D><<<L.blocks, 256, 0, L.stream>>>(T, fd.seed);
+  go(k_plan, 1, 32, 0, T, fd.ratio);
+  go(k_activate<D>, L.blocks, 256, 0, T, fd.seed);
   mark(KT_ACTIVATE);
-  k_pick<D><<<L.blocks, 256, 0, L.stream>>>(T, tu.thin);
+  go(k_pick<D>, L.blocks, 256, 0, T, tu.thin);
   mark(KT_PICK);
   if (tu.thin > 0) {
-    k_thin<D><<<L.blocks, 256, 0, L.stream>>>(T, tu.thin);
+    go(k_thin<D>, L.blocks, 256, 0, T, tu.thin);
     mark(KT_THIN);
   }
   // kernels with conflict tests come in two forms: exact tier on expansions
   // alone (small register allocation) or integer tier first (tu.exact_int)
   if (tu.exact_int)
-    k_cavity<D, 1><<<L.warps / 4, 128, 0, L.stream>>>(T, tu.adjacent, tu.big_block);
+    go(k_cavity<D, 1>, L.warps / 4, 128, 0, T, tu.adjacent, tu.big_block);
   else
-    k_cavity<D, 0><<<L.warps / 4, 128, 0, L.stream>>>(T, tu.adjacent, tu.big_block);
+    go(k_cavity<D, 0>, L.warps / 4, 128, 0, T, tu.adjacent, tu.big_block);
   mark(KT_CAVITY);
   // with big_block, searches that outgrew a warp's shared memory are redone
   // by whole blocks (the host turns it on once a call has spilled searches)
   if (tu.big_block) {
     if (tu.exact_int)
-      k_cavity_big<D, 1><<<g_big_grid, 512, kBigSmem, L.stream>>>(T, tu.adjacent);
+      go(k_cavity_big<D, 1>, g_big_grid, 512, kBigSmem, T, tu.adjacent);
     else
-      k_cavity_big<D, 0><<<g_big_grid, 512, kBigSmem, L.stream>>>(T, tu.adjacent);
+      go(k_cavity_big<D, 0>, g_big_grid, 512, kBigSmem, T, tu.adjacent);
     mark(KT_BIG);
   }
   // the commit half needs little shared memory per warp and few registers,
@@ -2856,31 +2899,31 @@ void round_impl(const DevTree& T, const Launch& L, const Tuning& tu, const Feed&
     const int last = p == tu.passes - 1;
     if (p > 0) {
       // reclaim (73 registers, no shared memory) runs twice the search's warps
-      k_reclaim<D><<<L.warps / 2, 128, 0, L.stream>>>(T, p, tu.adjacent);
+      go(k_reclaim<D>, L.warps / 2, 128, 0, T, p, tu.adjacent);
       mark(KT_RECLAIM);
     }
     if (tu.adjacent) {
       if (tu.exact_int)
-        k_check<D, 1, 1><<<decide_grid, 128, 4 * sizeof(HeadBuf), L.stream>>>(T, p, last, fd.seed, 0);
+        go(k_check<D, 1, 1>, decide_grid, 128, 4 * sizeof(HeadBuf), T, p, last, fd.seed, 0);
       else
-        k_check<D, 1, 0><<<decide_grid, 128, 4 * sizeof(HeadBuf), L.stream>>>(T, p, last, fd.seed, 0);
+        go(k_check<D, 1, 0>, decide_grid, 128, 4 * sizeof(HeadBuf), T, p, last, fd.seed, 0);
       mark(KT_DECIDE);
-      k_check<D, 2, 0><<<commit_grid, 128, 4 * sizeof(WarpCommit<D>), L.stream>>>(T, p, last, fd.seed,
+      go(k_check<D, 2, 0>, commit_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed,
                                                                                   tu.big_block);
       mark(KT_CHECK);
       if (tu.big_block) {
-        k_commit_big<D><<<g_big_grid, 512, 0, L.stream>>>(T);
+        go(k_commit_big<D>, g_big_grid, 512, 0, T);
         mark(KT_BIGW);
       }
     } else {
       if (tu.exact_int)
-        k_check<D, 0, 1><<<strict_grid, 128, 4 * sizeof(WarpCommit<D>), L.stream>>>(T, p, last, fd.seed, 0);
+        go(k_check<D, 0, 1>, strict_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed, 0);
       else
-        k_check<D, 0, 0><<<strict_grid, 128, 4 * sizeof(WarpCommit<D>), L.stream>>>(T, p, last, fd.seed, 0);
+        go(k_check<D, 0, 0>, strict_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed, 0);
       mark(KT_CHECK);
     }
   }
-  k_relocate<D><<<L.blocks, 256, 0, L.stream>>>(T);
+  go(k_relocate<D>, L.blocks, 256, 0, T);
   mark(KT_RELOCATE);
 }
 

@@ -748,8 +748,8 @@ vd::Launch sized_launch(const vd_tree* t, int64_t items) {
 }
 
 // The graph of `chunk` rounds for these launches, or null when there is none
-// yet.  A chunk of several rounds that an earlier call has asked for is captured;
-// asked for the first time it is only noted.
+// yet: a chunk that an earlier call has asked for is captured, one asked for the
+// first time is only noted.
 vd_tree::ChunkGraph* chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Feed& fd) {
   vd_tree::ChunkGraph* hit = nullptr;
   for (auto& g : t->graphs)
@@ -782,7 +782,7 @@ vd_tree::ChunkGraph* chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, con
     hit = &t->graphs.back();
   }
   if (hit->exec) return hit;
-  if (chunk > 1 && hit->call == t->calls) return nullptr;
+  if (hit->call == t->calls) return nullptr;
   const long long before = vd::launches_total();
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -805,33 +805,25 @@ vd_tree::ChunkGraph* chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, con
   return hit;
 }
 
-// Launches `chunk` rounds as a CUDA graph: one of the whole chunk once an
-// earlier call has run such a chunk, until then a graph of one round replayed
-// `chunk` times.  Capturing 8 rounds costs about 0.3 ms and saves 20 us a
-// replay, so it does not pay within one call (one-shot 10,000 points 2D: 4.6 ms
-// of insertion with chunk graphs captured at once, 4.1 with one-round graphs,
-// repeated calls 3.1 and 3.3).  Returns false (nothing launched) when graphs are
-// off for this tree: profiling and tracing need per-kernel events, and a failed
-// capture turns graphs off.
+// Launches `chunk` rounds as one CUDA graph if an earlier call has run such a
+// chunk.  Capturing 8 rounds costs about 0.3 ms and saves 3 us a round against
+// early launches (Launch::early), so it does not pay within one call: inserting
+// 10,000 2D points into a new tree took 4.6 ms with every chunk captured at once,
+// 3.5 with one-round graphs, 3.3 with early launches, and 3.2 replayed; 300,000
+// 3D points 20.3 with one-round graphs, 20.0 with early launches.  Returns false
+// (nothing launched) when there is no graph yet or graphs are off for this tree:
+// profiling and tracing need per-kernel events, and a failed capture turns
+// graphs off.
 bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Feed& fd) {
   if (!t->use_graphs || t->prof || t->trace) return false;
   const vd_tree::ChunkGraph* g = chunk_graph(t, L, chunk, fd);
-  int replays = 1;
-  if (!g && t->use_graphs) {
-    g = chunk_graph(t, L, 1, fd);
-    replays = chunk;
-  }
   if (!g) return false;
-  for (int k = 0; k < replays; ++k) {
-    if (cudaGraphLaunch(g->exec, t->stream) != cudaSuccess) {
-      cudaGetLastError();
-      t->use_graphs = false;
-      if (k == 0) return false;
-      for (; k < replays; ++k) vd::launch_round(t->T, L, t->dim, t->tuning, fd, nullptr);
-      return true;
-    }
-    vd::note_launches(g->launches);
+  if (cudaGraphLaunch(g->exec, t->stream) != cudaSuccess) {
+    cudaGetLastError();
+    t->use_graphs = false;
+    return false;
   }
+  vd::note_launches(g->launches);
   return true;
 }
 
@@ -883,8 +875,10 @@ int run_rounds(vd_tree* t, int& r, int64_t n_call, uint64_t seed) {
       const double grow = std::pow(1.4, chunk);
       const int64_t est = std::min<int64_t>(n_call - fed + active,
                                             (int64_t)((double)(done + active + 256) * grow));
-      const vd::Launch L = sized_launch(t, est);
-      if (!launch_chunk_graph(t, L, chunk, fd))
+      vd::Launch L = sized_launch(t, est);
+      const bool replayed = launch_chunk_graph(t, L, chunk, fd);
+      L.early = true;
+      if (!replayed)
         for (int k = 0; k < chunk; ++k) vd::launch_round(t->T, L, t->dim, t->tuning, fd, round_prof(t, k));
       r += chunk;
     }
