@@ -164,7 +164,10 @@ __global__ void __launch_bounds__(256) k_edge_uniq(int n_in, const int* off, int
   for (int u = blockIdx.x * 8 + w; u < n_in; u += gridDim.x * 8) {
     const int b = off[u], L = off[u + 1] - b;
     if (L > kWarpSeg) {
-      if (lane == 0) big[atomicAdd(nbig, 1)] = u;
+      if (lane == 0) {
+        big[atomicAdd(nbig, 1)] = u;
+        ucnt[u] = 0;  // placed once k_edge_uniq_big has counted it
+      }
       continue;
     }
     if (L <= 1) {
