@@ -884,6 +884,13 @@ int run_rounds(vd_tree* t, int& r, int64_t n_call, uint64_t seed) {
     }
     rc = sync_counters(t);
     if (rc) break;
+    if (h.wasted > 0) {
+      // allocations that did not fit are the last ones counted: without them
+      // the count is of slots that exist again, whichever way this call ends
+      h.nsimp -= h.wasted;
+      h.wasted = 0;
+      cudaMemcpyAsync(t->T.ctr, &h, sizeof(Counters), cudaMemcpyHostToDevice, t->stream);
+    }
     if (ran_small)
       r = h.round + 1;  // the kernel decided how many rounds it ran
     else
@@ -921,8 +928,6 @@ int run_rounds(vd_tree* t, int& r, int64_t n_call, uint64_t seed) {
     // grow pools when a round had to defer work
     bool fix = false;
     if (h.simp_overflow || (double)h.nsimp > 0.85 * t->T.cap_simp) {
-      h.nsimp -= h.wasted;
-      h.wasted = 0;
       h.simp_overflow = 0;
       int64_t want = (int64_t)t->T.cap_simp + std::max<int64_t>(t->T.cap_simp / 2, 4096);
       rc = ensure_simplices(t, want);
