@@ -2212,6 +2212,12 @@ __global__ void __launch_bounds__(128) k_rounds_small(DevTree T, Tuning tu, unsi
 // another error code, or -1 when the region outgrew the warp's shared memory
 // and nothing but the point record was written (the caller then inserts it
 // through the rounds).
+// One warp's chain of dependent loads bounds it, not bandwidth: a call on a tree of
+// 500 to 3,000 3D points took 41 us with an FP64 test against the super simplex,
+// the hint levels read one after another and the walk run to the simplex that
+// contains the point; 36.7 us with FP32 signs there, one round trip for all levels
+// and the walk stopped by the first stored sphere that certainly holds the point
+// (an empty launch and the copy of the counters are 9.5 us of either).
 template <int D>
 __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y, double z, int vid) {
   constexpr int NV = D + 1;
@@ -2241,19 +2247,27 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
     if (s_status == 0) {
       reinterpret_cast<double4_32a*>(T.pts)[vid] = make_double4_32a(c[0], c[1], c[2], 0.0);
       T.ptf[vid] = fq;
-      const SetGeo& g = T.sets[0];
-      vdp::VPt sv[NV];
-      for (int j = 0; j < NV; ++j) sv[j] = load_pt(T, g.sup[j]);
-      const vdp::VPt p{c[0], c[1], c[2], 0.0};
-      if (vdp::exit_face<D, true>(sv, p, (1u << NV) - 1, tl, perr) >= 0) s_status = E_OUTSIDE;
     }
     if (s_status == 0) {
-      // walk from the finest hint of the point's cell (as k_activate)
+      // the hints of the point's cell on every level and the super vertices in
+      // one round trip; the walk starts at the finest hint (as k_activate)
       const SetGeo& g = T.sets[0];
       int ic[3];
       hint_cell<D>(g, fq, ic);
+      int hv[kHintLevelsMax + 1];
+#pragma unroll
+      for (int l = 0; l <= kHintLevelsMax; ++l) hv[l] = l <= g.hint_levels ? T.hint[hint_at<D>(g, ic, l)] : -1;
+      vdp::FPt sf[NV];
+      for (int j = 0; j < NV; ++j) sf[j] = load_fpt(T, g.sup[j]);
+      auto load_sup = [&](vdp::VPt* v64, vdp::VPt& p64) {
+        for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, g.sup[j]);
+        p64 = vdp::VPt{c[0], c[1], c[2], 0.0};
+      };
+      if (vdp::exit_face_hl<D, true>(sf, fq, (1u << NV) - 1, tl, perr, load_sup) >= 0) s_status = E_OUTSIDE;
       int cur = -1;
-      for (int l = g.hint_levels; l >= 0 && cur < 0; --l) cur = T.hint[hint_at<D>(g, ic, l)];
+#pragma unroll
+      for (int l = kHintLevelsMax; l >= 0; --l)
+        if (cur < 0) cur = hv[l];
       if (cur < 0) cur = g.root;
       int4 v, nn;
       load_simplex(T, cur, v, nn);
@@ -2265,9 +2279,18 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
         }
         load_simplex(T, cur, v, nn);
       }
+      // the walk may end before the simplex that contains the point, at one
+      // whose stored sphere certainly holds it (3D): the region is connected,
+      // and such a point equals no vertex, since no vertex lies inside a sphere
       int step = 0;
       const int cap = 1 << 16;
+      bool inside = false;
       for (; s_status == 0 && step < cap; ++step) {
+        if constexpr (D == 3) {
+          const float4 sp = *reinterpret_cast<const float4*>(T.sph + cur);
+          inside = vdp::sphere_side<D>(vdp::Sph{sp.x, sp.y, sp.z, sp.w}, fq) > 0;
+          if (inside) break;
+        }
         vdp::FPt fv[NV];
         for (int j = 0; j < NV; ++j) fv[j] = load_fpt(T, get4(v, j));
         auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
@@ -2285,7 +2308,7 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
         load_simplex(T, cur, v, nn);
       }
       if (step == cap) s_status = E_WALK;
-      if (s_status == 0) {
+      if (s_status == 0 && !inside) {
         // a duplicate of a vertex of its simplex is skipped and recorded
         const vdp::VPt q{c[0], c[1], c[2], 0.0};
         int dup = -1;
