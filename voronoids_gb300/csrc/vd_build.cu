@@ -2414,6 +2414,504 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
 }
 
 // ---------------------------------------------------------------------------
+// The last points of a call, without rounds.
+//
+// A round is about ten dependent launches however few points are active, and the
+// points left when everything has been fed conflict with one another, so half of
+// them or fewer win a round: 14 rounds and 2 ms for the last 20,000 points of a
+// 1M-point build.  Here one warp takes one point after another and inserts it
+// under locks.  A warp locks every simplex before it reads it for good: the
+// conflict region and the simplices around it (whose links change).  A lock holds
+// the key of its point, and a lower key takes it over; before a warp writes, it
+// turns each of its locks, if it is still its own, into one that nobody takes.
+// So two insertions that write have disjoint locked sets, any order of them is an
+// order of single insertions, and the triangulation is the one the rounds would
+// build; and the lowest key around is never held up by the others.  What a warp
+// read before it lost a lock may be anything: every index in it is checked, and
+// nothing is written from it.  No warp ever waits for another: a lock that a lower
+// key or a writer holds ends the attempt, the warp gives back its own and tries
+// again a little later, kFinishTries times at most.  A point that is not inserted
+// then, one that equals a vertex, or one whose region does not fit in shared
+// memory stays for the rounds (k_refit gives it its simplex again).
+//
+// Lock of slot s: T.thin[s] equal to epoch(round) of the round that has not run
+// yet (being written), or that + 1 + the point's place in the list: lower than any
+// claim before it; free again is ~0.  Records are read past L1 (other warps change
+// them while this kernel runs).  The walk reads without locks: what it finds is
+// only where to begin, and under the lock the start is tested again.
+//
+// Bounded by the longest chain of points that conflict one with the next (20 to 40
+// us an insertion: locks, records and spheres are three round trips for every 32
+// faces), so neither the number of warps (4 to 16 an SM) nor the pause between
+// attempts matters: 3,000 last points of 10,000 in 2D 0.55 ms against 1.1 ms of
+// rounds, of 100,000 in 3D 1.0 against 1.6.  With locks that are never taken over,
+// points that block each other held up all around them: 450 of the 3,056 were not
+// in after 64 attempts each.
+constexpr int kFinishTries = 256;
+constexpr int kFinishWalk = 1024;  // steps of one attempt's walk, at most
+
+template <int D>
+struct FinishSet {
+  // region and surrounding simplices: at most MAXC + MAXF keys
+  static constexpr int HS = D == 3 ? 512 : 256;
+  static constexpr int ML = Cap<D>::MAXC + Cap<D>::MAXF;
+  int key[HS];
+  int in[HS];  // 1 in conflict, 2 not
+  int lock[ML];
+  int nlock;
+};
+
+// Slot of `key` in the set; fresh: this lane has added it.  -1: full.
+template <int D>
+__device__ int fset_add(FinishSet<D>& H, int key, bool& fresh) {
+  unsigned h = ((unsigned)key * 2654435761u) & (FinishSet<D>::HS - 1);
+  fresh = false;
+  for (int probe = 0; probe < FinishSet<D>::HS; ++probe) {
+    const int old = atomicCAS(&H.key[h], -1, key);
+    if (old == -1 || old == key) {
+      fresh = old == -1;
+      return (int)h;
+    }
+    h = (h + 1) & (FinishSet<D>::HS - 1);
+  }
+  return -1;
+}
+
+__device__ __forceinline__ void load_simplex_cg(const DevTree& T, int s, int4& v, int4& n) {  // s is in range
+  const int4* p = reinterpret_cast<const int4*>(T.simp + s);
+  v = __ldcg(p);
+  n = __ldcg(p + 1);
+}
+template <int D>
+__device__ __forceinline__ bool bad_record(const DevTree& T, int4 v) {
+  bool bad = false;
+  for (int j = 0; j <= D; ++j) bad = bad || bad_vert(T, get4(v, j));
+  return bad;
+}
+template <int D>
+__device__ __forceinline__ int sphere_tier_cg(const DevTree& T, int s, const vdp::FPt& fq) {
+  if (D != 3) return 0;
+  const float4 sp = __ldcg(reinterpret_cast<const float4*>(T.sph + s));
+  return vdp::sphere_side<D>(vdp::Sph{sp.x, sp.y, sp.z, sp.w}, fq);
+}
+
+// Walk of one lane from slot `cur` towards point vid, without locks.  Ends at a
+// simplex that seems to hold the point (or its sphere does); -1: led nowhere.
+template <int D>
+__device__ int finish_walk(const DevTree& T, int cur, int vid, const vdp::FPt& fq, vdp::Tally& tl, int& perr,
+                           unsigned& walk) {
+  constexpr int NV = D + 1;
+  for (int step = 0; step < kFinishWalk; ++step) {
+    if (bad_simp(T, cur)) return -1;
+    int4 v, n;
+    load_simplex_cg(T, cur, v, n);
+    if (v.x < 0) {  // removed: on to its star
+      if (n.x < 0) return -1;
+      cur = n.x >> 2;
+      continue;
+    }
+    if (bad_record<D>(T, v)) return -1;
+    if (D == 3 && sphere_tier_cg<D>(T, cur, fq) > 0) return cur;
+    vdp::FPt fv[NV];
+    for (int j = 0; j < NV; ++j) fv[j] = load_fpt(T, get4(v, j));
+    auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
+      for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, get4(v, j));
+      p64 = load_pt(T, vid);
+    };
+    const int f = vdp::exit_face_hl<D>(fv, fq, (1u << NV) - 1, tl, perr, load64);
+    if (f < 0) return cur;
+    const int code = get4(n, f);
+    if (code < 0) return -1;
+    cur = code >> 2;
+    ++walk;
+  }
+  return -1;
+}
+
+// Under the lock of `s`: 1 the point is certainly in conflict with it and equals no
+// vertex, 0 it is not the simplex to begin at, -1 the point equals a vertex.
+template <int D>
+__device__ int finish_start(const DevTree& T, int s, int4 v, int vid, const vdp::FPt& fq, vdp::Tally& tl, int& perr) {
+  constexpr int NV = D + 1;
+  if (v.x < 0 || bad_record<D>(T, v)) return 0;
+  if (D == 3 && sphere_tier_cg<D>(T, s, fq) > 0) return 1;
+  vdp::FPt fv[NV];
+  for (int j = 0; j < NV; ++j) fv[j] = load_fpt(T, get4(v, j));
+  auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
+    for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, get4(v, j));
+    p64 = load_pt(T, vid);
+  };
+  if (vdp::exit_face_hl<D>(fv, fq, (1u << NV) - 1, tl, perr, load64) >= 0) return 0;
+  const vdp::VPt q = load_pt(T, vid);
+  for (int j = 0; j < NV; ++j)
+    if (same_point_bits(load_pt(T, get4(v, j)), q)) return -1;
+  return 1;
+}
+
+enum : int { FIN_DONE = 0, FIN_AGAIN = 1, FIN_LEAVE = 2 };
+
+// One attempt of a warp to insert point vid, its walk starting at slot `cur` (all
+// lanes; set to where the next attempt should start).
+template <int D, int XT>
+__device__ int finish_try(const DevTree& T, WarpCommit<D>& W, FinishSet<D>& H, int* cav, int4* cn, int* F, int vid,
+                          int place, const vdp::FPt& fq, int& cur, int& id0, int& ncav_out, int& nfac_out, vdp::Tally& tl,
+                          int& perr, unsigned& ntests, unsigned& walk, int lane) {
+  constexpr int NV = D + 1;
+  constexpr int MAXC = Cap<D>::MAXC, MAXF = Cap<D>::MAXF;
+  Counters* ctr = T.ctr;
+  const unsigned long long lk = epoch(ctr->round + 1), mine = lk + 1 + (unsigned)place;
+  for (int i = lane; i < FinishSet<D>::HS; i += 32) H.key[i] = -1;
+  if (lane == 0) H.nlock = 0;
+  __syncwarp();
+  int st = FIN_AGAIN, begin = cur;
+  if (lane == 0) {
+    begin = finish_walk<D>(T, cur, vid, fq, tl, perr, walk);
+    if (begin >= 0 && atomicMin(T.thin + begin, mine) > mine) {
+      H.lock[0] = begin;
+      H.nlock = 1;
+      __threadfence();
+      int4 v, n;
+      load_simplex_cg(T, begin, v, n);
+      const int s = finish_start<D>(T, begin, v, vid, fq, tl, perr);
+      if (s > 0) {
+        cav[0] = begin;
+        cn[0] = n;
+        bool fresh;
+        H.in[fset_add<D>(H, begin, fresh)] = 1;
+        st = FIN_DONE;
+      } else if (s < 0) {
+        st = FIN_LEAVE;
+      }
+    }
+  }
+  st = __shfl_sync(FULL, st, 0);
+  begin = __shfl_sync(FULL, begin, 0);
+  if (begin >= 0) cur = begin;
+  __syncwarp();
+  // the region, breadth first, 32 (simplex, face) items at a time
+  int ncav = 1, nfac = 0, done = 0;
+  while (st == FIN_DONE && done < ncav * NV) {
+    const int it = done + lane, k = it / NV, f = it - k * NV;
+    const bool act = it < ncav * NV;
+    int code = -1, o = 0, h = -1, my = FIN_DONE;
+    bool fresh = false, in = false;
+    int4 v = make_int4(-1, -1, -1, -1), n = v;
+    if (act) {
+      code = get4(cn[k], f);
+      if (code >= 0) {
+        o = code >> 2;
+        if (bad_simp(T, o)) {
+          my = FIN_AGAIN;  // a lock was lost
+        } else {
+          h = fset_add<D>(H, o, fresh);
+          if (h < 0) my = FIN_LEAVE;
+        }
+      }
+    }
+    if (fresh) {
+      if (atomicMin(T.thin + o, mine) < mine) {
+        my = FIN_AGAIN;
+      } else {
+        const int i = atomicAdd(&H.nlock, 1);  // <= keys of the set
+        if (i < FinishSet<D>::ML) {
+          H.lock[i] = o;
+        } else {  // no room to remember it: given back at once
+          atomicCAS(T.thin + o, mine, ~0ull);
+          my = FIN_LEAVE;
+        }
+      }
+    }
+    st = (int)__reduce_max_sync(FULL, (unsigned)my);
+    if (st != FIN_DONE) break;
+    if (fresh) {
+      __threadfence();
+      load_simplex_cg(T, o, v, n);
+      if (v.x < 0 || bad_record<D>(T, v)) {
+        my = FIN_AGAIN;  // a live simplex links only live ones: a lock was lost
+      } else {
+        const int side = sphere_tier_cg<D>(T, o, fq);
+        ++ntests;
+        if (side != 0) ++tl.f32;
+        in = side > 0 || (side == 0 && conflict_tiers<D, XT>(T, v, fq, vid, tl, perr));
+        H.in[h] = in ? 1 : 2;
+      }
+    }
+    const unsigned add = __ballot_sync(FULL, in);
+    if (in) {
+      const int c = ncav + __popc(add & ((1u << lane) - 1));
+      if (c < MAXC) {
+        cav[c] = o;
+        cn[c] = n;
+      } else {
+        my = FIN_LEAVE;
+      }
+    }
+    __syncwarp();
+    const bool facet = act && (code < 0 || H.in[h] == 2);
+    const unsigned fm = __ballot_sync(FULL, facet);
+    if (facet) {
+      const int j = nfac + __popc(fm & ((1u << lane) - 1));
+      if (j >= MAXF) {
+        my = FIN_LEAVE;
+      } else if (code < 0) {
+        int4 kv, kn;
+        load_simplex_cg(T, cav[k], kv, kn);
+        put_facet(F, j, set4(kv, f, vid), code, (k << 4) | (f << 2) | f);
+      } else {
+        int4 ov, on;
+        load_simplex_cg(T, o, ov, on);
+        put_facet(F, j, facet_simplex<D>(ov, code & 3, vid), code, (k << 4) | ((code & 3) << 2) | f);
+      }
+    }
+    st = (int)__reduce_max_sync(FULL, (unsigned)my);
+    done = min(done + 32, ncav * NV);
+    ncav += __popc(add);
+    nfac += __popc(fm);
+  }
+  __syncwarp();
+  int base = 0, fresh_n = 0;
+  const int nl = min(H.nlock, FinishSet<D>::ML);
+  // writing: only with every lock still in hand
+  unsigned kept = 0;  // bit k: lock lane + 32 k is turned
+  if (st == FIN_DONE) {
+    bool all = true;
+    for (int i = lane, bit = 0; i < nl; i += 32, ++bit) {
+      if (atomicCAS(T.thin + H.lock[i], mine, lk) == mine) kept |= 1u << bit;
+      else all = false;
+    }
+    if (!__all_sync(FULL, all)) st = FIN_AGAIN;
+  } else {
+    for (int i = lane; i < nl; i += 32) atomicCAS(T.thin + H.lock[i], mine, ~0ull);
+  }
+  if (st == FIN_DONE) {
+    fresh_n = max(0, nfac - ncav);
+    if (lane == 0 && fresh_n > 0) {
+      base = atomicAdd(&ctr->nsimp, fresh_n);
+      if (base + fresh_n > T.cap_simp) {
+        atomicAdd(&ctr->wasted, fresh_n);
+        atomicExch(&ctr->simp_overflow, 1);
+        base = -1;
+      }
+    }
+    base = __shfl_sync(FULL, base, 0);
+    if (base < 0) {
+      st = FIN_LEAVE;
+      fresh_n = 0;
+    }
+  }
+  if (st == FIN_DONE) {
+    // a fresh slot is locked before any link leads to it
+    for (int i = lane; i < fresh_n; i += 32) __stcg(T.thin + base + i, lk);
+    // slots as in k_insert_one
+    for (int i = lane; i < ncav; i += 32) W.first[i] = 0x7fffffff;
+    __syncwarp();
+    for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[rec_k(F[6 * j + 5])], j);
+    __syncwarp();
+    int nfree = 0;
+    for (int i0 = 0; i0 < ncav; i0 += 32) {
+      const int i = i0 + lane;
+      const bool fr = i < ncav && W.first[i] == 0x7fffffff;
+      const unsigned m = __ballot_sync(FULL, fr);
+      if (fr) W.freeslot[nfree + __popc(m & ((1u << lane) - 1))] = cav[i];
+      nfree += __popc(m);
+    }
+    int nsec = 0;
+    for (int j0 = 0; j0 < nfac; j0 += 32) {
+      const int j = j0 + lane;
+      int id = 0;
+      bool sec = false;
+      if (j < nfac) {
+        const int k = rec_k(F[6 * j + 5]);
+        sec = W.first[k] != j;
+        if (!sec) id = cav[k];
+      }
+      const unsigned m = __ballot_sync(FULL, sec);
+      if (sec) {
+        const int t = nsec + __popc(m & ((1u << lane) - 1));
+        id = t < nfree ? W.freeslot[t] : base + (t - nfree);
+      }
+      if (j < nfac) W.id[j] = id;
+      nsec += __popc(m);
+    }
+    __threadfence();
+    __syncwarp();
+    id0 = W.id[0];
+    for (int t = nsec + lane; t < nfree; t += 32)
+      store_simplex(T, W.freeslot[t], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
+    // no slot carries round -2 in `killed`, so every outer neighbour is repointed
+    write_star<D, D == 3>(T, W, F, nfac, vid, -2, lane);
+    ncav_out = ncav;
+    nfac_out = nfac;
+  }
+  // what was written is visible before the locks are free
+  __threadfence();
+  __syncwarp();
+  __threadfence();
+  for (int i = lane, bit = 0; i < nl; i += 32, ++bit)
+    if ((kept >> bit) & 1u) __stcg(T.thin + H.lock[i], ~0ull);
+  for (int i = lane; i < fresh_n; i += 32) __stcg(T.thin + base + i, ~0ull);
+  __syncwarp();
+  return st;
+}
+
+template <int D, int XT>
+__global__ void __launch_bounds__(32) k_finish(DevTree T) {
+  constexpr int HR = WarpCommit<D>::HR;
+  __shared__ WarpCommit<D> W;
+  __shared__ FinishSet<D> H;
+  __shared__ int cav[Cap<D>::MAXC];
+  __shared__ int4 cn[Cap<D>::MAXC];
+  __shared__ __align__(16) int F[6 * Cap<D>::MAXF];
+  const int lane = threadIdx.x;
+  Counters* ctr = T.ctr;
+  const int par = (ctr->round + 1) & 1;
+  const int n = min(ctr->nact[par], T.cap_cand);
+  for (int i = lane; i < HR; i += 32) {
+    W.rk[i] = ~0ull;
+    W.ra[i] = -1;
+  }
+  __syncwarp();
+  vdp::Tally tl = {0, 0, 0, 0};
+  int perr = 0, nins = 0, maxc = 0, maxf = 0;
+  unsigned ntests = 0, walk = 0;
+  unsigned long long created = 0, killed = 0, holes = 0;
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int4 e = T.act[par][i];
+    if (e.x < 0) continue;
+    const vdp::FPt fq = load_fpt(T, e.x);
+    int cur = e.y, id0 = 0, ncav = 0, nfac = 0, st = FIN_AGAIN;
+    for (int a = 0; a < kFinishTries && st == FIN_AGAIN; ++a) {
+      if (a > 0) {
+        // about 2 us, a tenth of an insertion (a quarter or four times as long: the same)
+        __nanosleep(100 + (((unsigned)e.x * 0x9E3779B1u + (unsigned)a * 0x85EBCA77u) >> 20));
+      }
+      st = finish_try<D, XT>(T, W, H, cav, cn, F, e.x, i, fq, cur, id0, ncav, nfac, tl, perr, ntests, walk, lane);
+    }
+    if (lane == 0) {
+      if (st == FIN_DONE) {
+        write_hints<D>(T, e.x, fq, id0);
+        ++nins;
+        created += nfac;
+        killed += ncav;
+        holes += max(0, ncav - nfac);
+        maxc = max(maxc, ncav);
+        maxf = max(maxf, nfac);
+      } else {
+        T.act[par ^ 1][atomicAdd(&ctr->nleft, 1)] = e;
+      }
+    }
+    __syncwarp();
+  }
+  if (perr) set_error(ctr, E_PRECISION);
+  flush_tally(ctr, tl, ntests, walk);
+  if (lane == 0 && nins > 0) {
+    atomicAdd(&ctr->ninserted, nins);
+    atomicAdd(&ctr->winners, nins);
+    atomicAdd(&ctr->created, created);
+    atomicAdd(&ctr->killed, killed);
+    if (holes) atomicAdd(&ctr->holes, (int)holes);
+    atomicMax(&ctr->max_cav, maxc);
+    atomicMax(&ctr->max_fac, maxf);
+  }
+}
+
+// Before k_finish, one block: active points that equal one another are left for
+// the rounds, which insert the one of the best priority.  At most kFinishMax points.
+constexpr int kTwinSlots = 2 * kFinishMax;
+__global__ void __launch_bounds__(1024) k_twins(DevTree T) {
+  __shared__ int tab[kTwinSlots];
+  __shared__ unsigned char twin[kFinishMax];
+  Counters* ctr = T.ctr;
+  const int par = (ctr->round + 1) & 1;
+  const int n = min(min(ctr->nact[par], T.cap_cand), kFinishMax);
+  for (int i = threadIdx.x; i < kTwinSlots; i += blockDim.x) tab[i] = -1;
+  for (int i = threadIdx.x; i < kFinishMax; i += blockDim.x) twin[i] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const vdp::VPt q = load_pt(T, T.act[par][i].x);
+    // -0 and 0 are one value
+    const unsigned long long m = (unsigned long long)__double_as_longlong(q.x + 0.0) * 0x9E3779B97F4A7C15ull ^
+                                 (unsigned long long)__double_as_longlong(q.y + 0.0) * 0xC2B2AE3D27D4EB4Full ^
+                                 (unsigned long long)__double_as_longlong(q.z + 0.0) * 0x165667B19E3779F9ull;
+    unsigned h = (unsigned)((m ^ (m >> 29)) * 0x9E3779B97F4A7C15ull >> 40) & (kTwinSlots - 1);
+    for (int probe = 0; probe < kTwinSlots; ++probe, h = (h + 1) & (kTwinSlots - 1)) {
+      const int j = atomicCAS(&tab[h], -1, i);
+      if (j < 0) break;
+      if (same_point_bits(load_pt(T, T.act[par][j].x), q)) {
+        twin[i] = 1;
+        twin[j] = 1;
+        break;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    if (twin[i]) {
+      T.act[par ^ 1][atomicAdd(&ctr->nleft, 1)] = T.act[par][i];
+      T.act[par][i].x = -1;
+    }
+}
+
+// After k_finish, one block: the points it left become the active list of the next
+// round again, each walking from its old slot to the simplex that contains it.
+template <int D>
+__global__ void __launch_bounds__(256) k_refit(DevTree T) {
+  constexpr int NV = D + 1;
+  Counters* ctr = T.ctr;
+  const int round = ctr->round + 1, par = round & 1;
+  const int n = ctr->nleft;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ctr->nact[par] = 0;
+    ctr->nleft = 0;
+  }
+  __syncthreads();
+  vdp::Tally tl = {0, 0, 0, 0};
+  int perr = 0;
+  unsigned walk = 0;
+  for (int b = 0; b < n; b += blockDim.x) {
+    const int i = b + threadIdx.x;
+    const bool act = i < n;
+    int4 e = make_int4(-1, 0, 0, 0);
+    if (act) {
+      e = T.act[par ^ 1][i];
+      const vdp::FPt fp = load_fpt(T, e.x);
+      int4 v, nn;
+      load_simplex(T, e.y, v, nn);
+      const int cap = 1 << 16;
+      int step = 0;
+      for (; step < cap; ++step) {
+        int f = 0;
+        if (v.x >= 0) {
+          vdp::FPt fv[NV];
+          for (int j = 0; j < NV; ++j) fv[j] = load_fpt(T, get4(v, j));
+          auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
+            for (int j = 0; j < NV; ++j) v64[j] = load_pt(T, get4(v, j));
+            p64 = load_pt(T, e.x);
+          };
+          f = vdp::exit_face_hl<D>(fv, fp, (1u << NV) - 1, tl, perr, load64);
+          if (f < 0) break;
+        }
+        const int code = get4(nn, f);  // a dead slot's first entry leads into its star
+        if (code < 0 || bad_simp(T, code >> 2)) {
+          set_error(ctr, E_INTERNAL);
+          break;
+        }
+        e.y = code >> 2;
+        load_simplex(T, e.y, v, nn);
+        ++walk;
+      }
+      if (step == cap) set_error(ctr, E_WALK);
+    }
+    vote_min(T.vote, act, e.y, epoch(round) | (unsigned)e.z);
+    const int k = warp_append(&ctr->nact[par], act);
+    if (act) T.act[par][k] = e;
+  }
+  if (perr) set_error(ctr, E_PRECISION);
+  flush_tally(ctr, tl, 0, walk);
+}
+
+// ---------------------------------------------------------------------------
 // The first points of a fresh single-set build, one after another in one
 // block, with the whole triangulation in shared memory.
 //
@@ -3090,6 +3588,20 @@ void launch_insert_one(const DevTree& T, cudaStream_t stream, int dim, const dou
     k_insert_one<2><<<1, 32, 0, stream>>>(T, c[0], c[1], 0.0, vid);
 }
 
+void launch_finish(const DevTree& T, const Launch& L, int dim, bool exact_int) {
+  note_launches(3);
+  k_twins<<<1, 1024, 0, L.stream>>>(T);
+  if (dim == 3) {
+    if (exact_int) k_finish<3, 1><<<L.blocks, 32, 0, L.stream>>>(T);
+    else k_finish<3, 0><<<L.blocks, 32, 0, L.stream>>>(T);
+    k_refit<3><<<1, 256, 0, L.stream>>>(T);
+  } else {
+    if (exact_int) k_finish<2, 1><<<L.blocks, 32, 0, L.stream>>>(T);
+    else k_finish<2, 0><<<L.blocks, 32, 0, L.stream>>>(T);
+    k_refit<2><<<1, 256, 0, L.stream>>>(T);
+  }
+}
+
 void launch_round(const DevTree& T, const Launch& L, int dim, const Tuning& tu, const Feed& fd, Prof* pf) {
   if (dim == 3)
     round_impl<3>(T, L, tu, fd, pf);
@@ -3100,6 +3612,6 @@ void launch_round(const DevTree& T, const Launch& L, int dim, const Tuning& tu, 
 const char* const kKernelTypeNames[KT_COUNT] = {"k_pick",     "k_thin",         "k_cavity",     "k_check",
                                                 "k_reclaim",  "k_relocate",     "k_activate",   "edges",
                                                 "k_decide",   "k_rounds_small", "k_cavity_big", "k_commit_big",
-                                                "k_seed"};
+                                                "k_seed",     "k_finish"};
 
 }  // namespace vd

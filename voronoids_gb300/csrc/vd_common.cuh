@@ -111,6 +111,7 @@ struct Counters {
   unsigned bar_count, bar_gen;
   int bar_abort, coop_go;
   int single;                       // outcome of the last one-point insertion (k_insert_one)
+  int nleft;                        // points that k_finish left for the rounds
 };
 
 // Sum of a striped statistics counter (host or device).
@@ -302,6 +303,7 @@ enum {
   KT_BIG,
   KT_BIGW,
   KT_SEED,
+  KT_FINISH,
   KT_COUNT
 };
 extern const char* const kKernelTypeNames[KT_COUNT];
@@ -326,6 +328,12 @@ void launch_round(const DevTree& T, const Launch& L, int dim, const Tuning& tu, 
 // its vertex id vid (the next one of the tree).  ctr->single receives the
 // outcome (see k_insert_one in vd_build.cu).
 void launch_insert_one(const DevTree& T, cudaStream_t stream, int dim, const double* c, int vid);
+// Most points that launch_finish takes.
+constexpr int kFinishMax = 4096;
+// The active points of the next round inserted one by one by L.blocks warps
+// under locks, without rounds (k_finish in vd_build.cu); those it leaves are the
+// active list again.
+void launch_finish(const DevTree& T, const Launch& L, int dim, bool exact_int);
 // The first `npts` points of `order` (the first `nlev` priority levels of a
 // fresh single-set call, priorities under `seed`) inserted one after another
 // by one block, the triangulation in shared memory (k_seed in vd_build.cu).
