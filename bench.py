@@ -39,10 +39,10 @@ N_POINTS = 1_000_000
 SEED = 0x5EED
 
 # Algorithmic bytes per unit: k_cavity moves one 32-byte simplex record and
-# four 32-byte split-coordinate records per conflict test; the decide half of
+# its 16-byte stored sphere per conflict test; the decide half of
 # the check reads a candidate's claims and lists (~1264 B) and the commit half
 # writes a winner's star (~1240 B).
-BYTES_PER_TEST_3D = 160
+BYTES_PER_TEST_3D = 48
 BYTES_PER_CHECK = 1264
 BYTES_PER_WIN = 1240
 
