@@ -566,7 +566,6 @@ __device__ __forceinline__ void pick_body(DevTree T, int thin, int bid, int nblk
     T.ctr->nact[par ^ 1] = 0;
     for (int k = 1; k < kStages; ++k) T.ctr->nwl[k] = 0;
     T.ctr->nwin = 0;
-    T.ctr->win_lo = 0;
   }
   const int n = T.ctr->nact[par];
   const unsigned long long ep = epoch(round);
@@ -1379,8 +1378,9 @@ __device__ __forceinline__ void ridge_of(const int* r, int g, int qf, int& r0, i
 // Writes one new simplex and repoints its outer neighbour.  An outer
 // neighbour that another winner of this round removed (adjacent mode) is left
 // alone: the two new simplices on that facet are linked at the start of
-// k_relocate (fix_body).
-template <int D, bool SPH>
+// k_relocate (fix_body).  TOUCH: the outer neighbour is marked as repointed, for
+// the strict mode's k_reclaim.
+template <int D, bool SPH, bool TOUCH>
 __device__ __forceinline__ bool emit_simplex(const DevTree& T, const int* r, int myid, int4 nn, int round,
                                              const vdp::FPt& fq) {
   const int4 v = make_int4(r[0], r[1], r[2], r[3]);
@@ -1390,7 +1390,7 @@ __device__ __forceinline__ bool emit_simplex(const DevTree& T, const int* r, int
   if (o < 0 || bad_simp(T, o >> 2)) return false;
   if (T.killed[o >> 2].x == round) return true;  // another winner's cavity: linked by fix_body
   reinterpret_cast<int*>(T.simp + (o >> 2))[4 + (o & 3)] = (myid << 2) | qf;
-  T.touched[o >> 2] = round;
+  if (TOUCH) T.touched[o >> 2] = round;
   return false;
 }
 
@@ -1407,7 +1407,7 @@ __device__ __forceinline__ unsigned ridge_hash(int r0, int r1) {
 }
 // Returns, per lane, a bit for each of its facets (j = lane, lane + 32, ...)
 // whose outer neighbour another winner of this round removed.
-template <int D, bool SPH>
+template <int D, bool SPH, bool TOUCH = false>
 __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __restrict__ FR, int nfac, int qv,
                                int round, int lane) {
   constexpr int NV = D + 1;
@@ -1420,7 +1420,7 @@ __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __
   for (int j = lane, bit = 0; j < nfac; j += 32, ++bit) {
     const int* r = FR + 6 * j;
     const int qf = rec_q(r[5]);
-    if (emit_simplex<D, SPH>(T, r, W.id[j], set4(make_int4(-1, -1, -1, -1), qf, r[4]), round, fq)) dead |= 1u << bit;
+    if (emit_simplex<D, SPH, TOUCH>(T, r, W.id[j], set4(make_int4(-1, -1, -1, -1), qf, r[4]), round, fq)) dead |= 1u << bit;
   }
   const int sweeps = (nfac * D / 2 + PER_SWEEP - 1) / PER_SWEEP;
   // the table is empty on entry (cleared when the warp starts, and after
@@ -1475,7 +1475,7 @@ __device__ unsigned write_star(const DevTree& T, WarpCommit<D>& W, const int* __
 // Star of one winner, large case: every (facet, face) inserts its ridge into
 // an open-addressing table (two halves per ridge), then reads its partner.
 // A warp (BLOCK = false) or the whole block (k_commit_big) writes it.
-template <int D, bool SPH, bool BLOCK = false>
+template <int D, bool SPH, bool BLOCK = false, bool TOUCH = false>
 __device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, int nfac, int qv, int round,
                                int* R, int lane) {
   constexpr int NV = D + 1;
@@ -1543,7 +1543,7 @@ __device__ void write_star_big(const DevTree& T, const int* FR, const int* ID, i
       }
       nn = set4(nn, g, (ID[m] << 2) | (other & 3));
     }
-    emit_simplex<D, SPH>(T, r, ID[j], nn, round, fq);
+    emit_simplex<D, SPH, TOUCH>(T, r, ID[j], nn, round, fq);
   }
   sync();
 }
@@ -1603,14 +1603,19 @@ __device__ __forceinline__ void publish_marked(const DevTree& T, int* F, const i
 // on that facet: then the two new simplices on the facet are locally
 // Delaunay and inserting both equals inserting them one after the other.
 // MODE 1 decides (claims, facet tests, fresh slots, kill marks) for all
-// candidates of the pass, so that MODE 2, which writes the stars, knows every
-// simplex removed in the pass and leaves links into them to fix_body.
+// candidates of the pass; MODE 2 writes the stars once all passes are decided,
+// knows every simplex removed in the round and leaves links into them to fix_body.
+// A later pass needs no star of an earlier one: k_reclaim drops a candidate whose
+// region or outer simplices were removed, and that is also every candidate with a
+// simplex whose link a star will change (its neighbour there was removed).  One
+// commit a round instead of one a pass: 1M 3D points 34.6 -> 32.9 ms, 100,000 13.0 ->
+// 12.3, 1M 2D points 14.6 -> 14.2 (a launch and about 11 us of a small round).
 template <int D, int MODE, int XT>
 __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsigned long long seed, int bid, int nblk,
                                            unsigned char* dsm, bool defer_big = false) {
   constexpr int NV = D + 1;
   const int round = T.ctr->round;
-  if (MODE == 1 && bid == 0 && threadIdx.x == 0) T.ctr->nbigw = 0;  // stars deferred by this pass's commit
+  if (MODE == 1 && bid == 0 && threadIdx.x == 0) T.ctr->nbigw = 0;  // stars deferred by the commit half
   const int sin = 2 * pass, sout = 2 * pass + 1;
   constexpr int MAXF = Cap<D>::MAXF, MAXC = Cap<D>::MAXC;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1636,11 +1641,9 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
   const int gw = bid * 4 + wib;
   int2 chunk = (MODE != 2 && gw < T.cap_wchunk) ? T.wchunk[gw] : make_int2(0, 0);
   const int nw = nblk * 4;
-  const int lo = MODE == 2 ? T.ctr->win_lo : 0;
-  if (MODE == 2 && bid == 0 && threadIdx.x == 0) T.ctr->win_sph = lo;
   const int nin = MODE == 2 ? T.ctr->nwin : T.ctr->nwl[sin];
   const int* list = MODE == 2 ? T.win : T.wl[sin & 1];
-  for (int it0 = lo + bid * 4 + wib; it0 < nin; it0 += 32 * nw) {
+  for (int it0 = bid * 4 + wib; it0 < nin; it0 += 32 * nw) {
     // lane k loads the list entry, state and candidate record of the warp's
     // k-th next item: one round trip for up to 32 items instead of three each
     const int nh = load_heads(T, H, list, it0, nin, nw, lane);
@@ -1784,7 +1787,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         // leftover cavity slots become holes pointing into the star
         for (int t = nsec + lane; t < nfree; t += 32)
           store_simplex(T, W.freeslot[t], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
-        dead = write_star<D, D == 3 && MODE != 2>(T, W, F, nfac, cd.x, round, lane);
+        dead = write_star<D, D == 3 && MODE != 2, MODE == 0>(T, W, F, nfac, cd.x, round, lane);
         small_star = true;
       } else {
         // large star (spilled search): plain slot assignment, ids in the
@@ -1803,7 +1806,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         IDS = ID;
         for (int i = nfac + lane; i < ncav; i += 32)
           store_simplex(T, P[i], make_int4(-1, -1, -1, -1), make_int4(id0 << 2, -1, -1, -1));
-        write_star_big<D, D == 3 && MODE != 2>(T, F, ID, nfac, cd.x, round, P + kOffR, lane);
+        write_star_big<D, D == 3 && MODE != 2, false, MODE == 0>(T, F, ID, nfac, cd.x, round, P + kOffR, lane);
       }
       if (MODE == 2) {
         // facets shared with another winner's cavity: publish this side's new
@@ -1922,8 +1925,8 @@ __global__ void __launch_bounds__(512, 1) k_commit_big(DevTree T) {
 // Stored spheres of the star of winner c (adjacent mode; a star of k_commit_big
 // has them already), by one warp.  Not in the commit half:
 // there the vertex loads and the sphere's arithmetic lie on every winner's path
-// (commit 7.1 -> 9.9 ms of the 1M-point build); the next kernel (k_reclaim, or
-// k_relocate after the last pass) has warps to spare for them.
+// (commit 7.1 -> 9.9 ms of the 1M-point build); k_relocate has warps to spare
+// for them.
 template <int D>
 __device__ __forceinline__ void star_spheres(const DevTree& T, int c, const int* F, int nfac, int lane) {
   const int qv = T.cand[c].x;
@@ -1940,13 +1943,12 @@ __device__ __forceinline__ void star_spheres(const DevTree& T, int c, const int*
 
 // Adjacent mode, end of a round: a new simplex whose outer neighbour another
 // winner removed takes, as that neighbour, the other winner's new simplex on
-// the same facet.  The last pass's stars get their spheres.
+// the same facet.  The round's stars get their spheres.
 template <int D>
 __device__ __forceinline__ void fix_body(DevTree T, int bid, int nblk) {
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nw = nblk * (blockDim.x >> 5);
   const int n = T.ctr->nwin;
-  const int sph = T.ctr->win_sph;
   const long long nrepl = 4LL * T.cap_simp;
   // the last warps of the grid take the winners, so that in a small round the
   // first warps, which relocate the points, do not wait for this chain first
@@ -1966,7 +1968,7 @@ __device__ __forceinline__ void fix_body(DevTree T, int bid, int nblk) {
       }
       reinterpret_cast<int*>(T.simp + id)[4 + g] = T.repl[o];
     }
-    if (D == 3 && it >= sph && !(info.y & kSpheresDone)) star_spheres<D>(T, c, F, nfac, lane);
+    if (D == 3 && !(info.y & kSpheresDone)) star_spheres<D>(T, c, F, nfac, lane);
   }
 }
 
@@ -1977,7 +1979,6 @@ __device__ __forceinline__ void fix_body(DevTree T, int bid, int nblk) {
 template <int D>
 __device__ __forceinline__ void reclaim_body(DevTree T, int pass, int adjacent, int bid, int nblk) {
   const int round = T.ctr->round;
-  if (bid == 0 && threadIdx.x == 0) T.ctr->win_lo = T.ctr->nwin;  // winners of this pass start here
   const int sin = 2 * pass - 1, sout = 2 * pass;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nc = min(T.ctr->ncand, T.cap_cand);
@@ -1996,7 +1997,8 @@ __device__ __forceinline__ void reclaim_body(DevTree T, int pass, int adjacent, 
     bool blocked = false;
     for (int i = lane; i < ncav; i += 32) {
       const int s = P[i];
-      blocked |= (T.killed[s].x == round) | (T.touched[s] == round);
+      blocked |= T.killed[s].x == round;
+      if (!adjacent) blocked |= T.touched[s] == round;
     }
     for (int j = lane; j < nfac; j += 32) {
       const int o = F[6 * j + 4];
@@ -2010,18 +2012,6 @@ __device__ __forceinline__ void reclaim_body(DevTree T, int pass, int adjacent, 
     if (lane == 0) {
       const int k = atomicAdd(&T.ctr->nwl[sout], 1);
       T.wl[sout & 1][k] = c;
-    }
-  }
-  if (D == 3 && adjacent) {
-    // spheres of the previous pass's stars, by the last warps first
-    const int n = T.ctr->nwin;
-    for (int i = T.ctr->win_sph + nw - 1 - (bid * 4 + wib); i < n; i += nw) {
-      const int c = T.win[i];
-      const int4 info = T.cinfo[c];
-      int *P, *F, ncav, nfac;
-      bool big;
-      cand_lists(T, info, P, F, ncav, nfac, big);
-      if (info.w == ST_DONE && !(info.y & kSpheresDone)) star_spheres<D>(T, c, F, nfac, lane);
     }
   }
 }
@@ -2179,11 +2169,13 @@ __global__ void __launch_bounds__(128) k_rounds_small(DevTree T, Tuning tu, unsi
       }
       if (tu.adjacent) {
         check_body<D, 1, 0>(T, p, last, seed, bid, nblk, dsm);
-        if (!grid_sync(c, nblk)) return;
-        check_body<D, 2, 0>(T, p, last, seed, bid, nblk, dsm);
       } else {
         check_body<D, 0, 0>(T, p, last, seed, bid, nblk, dsm);
       }
+      if (!grid_sync(c, nblk)) return;
+    }
+    if (tu.adjacent) {
+      check_body<D, 2, 0>(T, 0, 1, seed, bid, nblk, dsm);
       if (!grid_sync(c, nblk)) return;
     }
     relocate_body<D>(T, bid, nblk);
@@ -3383,8 +3375,8 @@ void round_impl(const DevTree& T, const Launch& L, const Tuning& tu, const Feed&
     cfg.numAttrs = L.early ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, args...);
   };
-  note_launches((tu.adjacent ? 6 + 3 * tu.passes - 1 : 6 + 2 * tu.passes - 1) - (tu.thin > 0 ? 0 : 1) +
-                (tu.big_block ? 1 + (tu.adjacent ? tu.passes : 0) : 0));
+  note_launches(6 + 2 * tu.passes - 1 + (tu.adjacent ? 1 : 0) - (tu.thin > 0 ? 0 : 1) +
+                (tu.big_block ? 1 + (tu.adjacent ? 1 : 0) : 0));
   go(k_plan, 1, 32, 0, T, fd.ratio);
   go(k_activate<D>, L.blocks, 256, 0, T, fd.seed);
   mark(KT_ACTIVATE);
@@ -3429,19 +3421,21 @@ void round_impl(const DevTree& T, const Launch& L, const Tuning& tu, const Feed&
       else
         go(k_check<D, 1, 0>, decide_grid, 128, 4 * sizeof(HeadBuf), T, p, last, fd.seed, 0);
       mark(KT_DECIDE);
-      go(k_check<D, 2, 0>, commit_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed,
-                                                                                  tu.big_block);
-      mark(KT_CHECK);
-      if (tu.big_block) {
-        go(k_commit_big<D>, g_big_grid, 512, 0, T);
-        mark(KT_BIGW);
-      }
     } else {
       if (tu.exact_int)
         go(k_check<D, 0, 1>, strict_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed, 0);
       else
         go(k_check<D, 0, 0>, strict_grid, 128, 4 * sizeof(WarpCommit<D>), T, p, last, fd.seed, 0);
       mark(KT_CHECK);
+    }
+  }
+  if (tu.adjacent) {
+    // the stars of every pass's winners
+    go(k_check<D, 2, 0>, commit_grid, 128, 4 * sizeof(WarpCommit<D>), T, 0, 1, fd.seed, tu.big_block);
+    mark(KT_CHECK);
+    if (tu.big_block) {
+      go(k_commit_big<D>, g_big_grid, 512, 0, T);
+      mark(KT_BIGW);
     }
   }
   go(k_relocate<D>, L.blocks, 256, 0, T);

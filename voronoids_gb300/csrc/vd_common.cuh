@@ -104,8 +104,7 @@ struct Counters {
   int nlev;                         // levels of the current call
   int feed_lo, feed_hi;             // range of `order` activated this round
   int round;                        // round being run (advanced by k_plan)
-  int nwin, win_lo;                 // winners of the round (adjacent mode), first of the pass
-  int win_sph;                      // first winner whose star has no stored spheres yet
+  int nwin;                         // winners of the round (adjacent mode)
   int max_levels;                   // deepest cavity search (breadth-first levels)
   // grid barrier and loop decision of the small-round kernel
   unsigned bar_count, bar_gen;
