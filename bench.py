@@ -883,7 +883,7 @@ def main():
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
                        "l2": "flushed between steps (256 MB write)", "edges": edges,
                        "tuning": "3D defaults: adjacent round mode, 2 resolution passes, thinning radius 2, "
-                                 "priority levels 64 x1.25 fed at 0.12 x inserted, rounds replayed as CUDA graphs"},
+                                 "priority levels 64 x1.4 fed at 0.12 x inserted, rounds replayed as CUDA graphs"},
             "clocks": clocks, "gpu_launches": int(launches), "e2e": e2e, "roofline": roof,
             "cpu_baseline": cpu,
             "build_stats": {k: stats[k] for k in ("rounds", "inserted", "max_cavity", "pred_f32", "pred_f64",

@@ -207,7 +207,7 @@ int vd_set_profiling(vd_tree* t, int on);
  * of a call are split by priority into levels of `first_prefix` points, then
  * growing by `growth` (1 < growth <= 16); a round activates further levels
  * while fewer than `ratio` (0 < ratio <= 64) times the inserted points are
- * active.  Defaults 64, 1.25 and 0.12. */
+ * active.  Defaults 64, 1.4 and 0.12. */
 int vd_set_schedule(vd_tree* t, int64_t first_prefix, double growth, double ratio);
 /* Round tuning: resolution passes per round (1..6) and the thinning radius
  * (0 = every nominee is searched, 1 = a nominee must hold its simplex and

@@ -163,7 +163,10 @@ struct vd_tree {
   // insertion schedule: priority levels from `first_prefix` points growing
   // by `growth`, fed while fewer than `ratio` x inserted points are active
   int64_t first_prefix = 64;
-  double growth = 1.25;
+  // (levels x1.25 / x1.4 / x1.6 / x2: 1M 3D points 33.0 / 32.7 / 33.5 / 34.2 ms, 300,000
+  // 18.1 / 17.6 / 17.3 / 17.5, 100,000 12.2 / 11.8 / 11.6 / 11.7, 1M 2D 14.2 / 13.7 / 13.9 /
+  // 13.9, 100,000 2D 5.2 / 4.9 / 5.1 / 4.8, 10,000 2D 2.73 / 2.69 / 2.61 / 2.54)
+  double growth = 1.4;
   double ratio = 0.12;
   int* d_counts = nullptr;     // 2 * kMaxLevels ints: level counts, cursors
   // profiling: per-kernel time from CUDA events on the tree's stream
