@@ -3526,17 +3526,22 @@ int prepare_once() {
 }
 }  // namespace
 
-// Once per process (trees may be created from several host threads).
 // Function attributes (dynamic shared memory above 48 KB) belong to a device's
-// context, so they are set once per device the process uses.
+// context, so they are set once per context the process uses on a device (trees
+// may be created from several host threads).
 int prepare_round_kernels() {
   constexpr int kMaxDevices = 64;
   static std::mutex mu;
   static int state[kMaxDevices] = {};  // 0 not yet, 1 ready, -1 failed
+  static unsigned long long context[kMaxDevices] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return E_CUDA;
   std::lock_guard<std::mutex> lock(mu);
-  if (state[dev] == 0) state[dev] = prepare_once() == E_OK ? 1 : -1;
+  unsigned long long id = context_id();
+  if (state[dev] == 0 || id == 0 || context[dev] != id) {
+    state[dev] = prepare_once() == E_OK ? 1 : -1;
+    context[dev] = context_id();  // prepare_once binds a context to a thread that has none
+  }
   return state[dev] == 1 ? E_OK : E_CUDA;
 }
 

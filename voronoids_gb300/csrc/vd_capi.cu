@@ -157,6 +157,7 @@ struct vd_tree {
   int64_t ncells = 0;
   // pinned staging for small host<->device copies
   unsigned long long* h_mm = nullptr;
+  unsigned long long pin_context = 0;  // context of the pinned block (hctr, h_mm, h_pair)
   // device staging of host input points (one-shot host path)
   double* d_in = nullptr;
   int64_t cap_in = 0;
@@ -465,7 +466,7 @@ void release(vd_tree* t) {
   dfree(t->T.wchunk, t->stream);
   t->h_mm = nullptr;
   dfree(t->d_in, t->stream);
-  if (t->hctr) vd::pinned_free(t->hctr);
+  if (t->hctr) vd::pinned_free(t->hctr, t->pin_context);
   t->hctr = nullptr;
   t->h_pair = nullptr;
   for (auto& p : t->profs)
@@ -526,7 +527,7 @@ int alloc_tree(vd_tree* t, int dim, void* stream) {
     t->own_stream = true;
   }
   // one pinned block: counters, then 8 keys, then 16 ints
-  char* pin = static_cast<char*>(vd::pinned_alloc());
+  char* pin = static_cast<char*>(vd::pinned_alloc(&t->pin_context));
   if (!pin) return vd::E_NOMEM;
   static_assert(vd::kPinnedBytes >= ((sizeof(Counters) + 15) & ~(size_t)15) + 8 * sizeof(unsigned long long) + 16 * sizeof(int),
                 "the pinned block holds them");

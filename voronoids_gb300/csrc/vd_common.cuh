@@ -235,15 +235,19 @@ __device__ inline int set_index(const DevTree& T, int vid) {
 }
 #endif
 
+// Id of the calling thread's current CUDA context (vd_memory.cu), 0 if none or
+// unknown.  No later context of the process has it again.
+unsigned long long context_id();
 // Memory (vd_memory.cu).  Device memory in stream order from a pool of the
-// library's own on the current device; null when there is none.  pool_free
+// library's own in the current context; null when there is none.  pool_free
 // takes null, and a stream that is gone.
 void* pool_alloc(size_t bytes, cudaStream_t st);
 void pool_free(void* p, cudaStream_t st);
-// Pinned host blocks of kPinnedBytes.
+// Pinned host blocks of kPinnedBytes; `context` is the context that a block
+// belongs to.
 constexpr size_t kPinnedBytes = 8192;
-void* pinned_alloc();
-void pinned_free(void* p);
+void* pinned_alloc(unsigned long long* context);
+void pinned_free(void* p, unsigned long long context);
 
 // Kernels launched by this library in this process (diagnostics).
 void note_launches(long long k);
@@ -316,8 +320,8 @@ struct Prof {
 };
 // Pool ints a warp of the region search takes at least at a time.
 int search_chunk_ints(int dim);
-// Kernel attributes the rounds need (shared-memory size); once per device
-// before the first round or capture.
+// Kernel attributes the rounds need (shared-memory size); once per context of a
+// device before the first round or capture.
 int prepare_round_kernels();
 // One insertion round; its number is kept on the device (Counters::round,
 // advanced by the round's first kernel), so a captured sequence of rounds

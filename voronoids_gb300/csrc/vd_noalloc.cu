@@ -250,9 +250,7 @@ __global__ void k_na_out(int nv, const int* S, uint2* out, long long cap) {
 // of the CUDA context it was looked up in.  The address belongs to the
 // module loaded in that context: after cudaDeviceReset (or any other end of
 // the device's primary context) the module is loaded again and the array may
-// sit elsewhere, so a new context id means a new lookup.  Context ids come
-// from the driver API (cuCtxGetCurrent, cuCtxGetId), reached through the
-// runtime's driver entry points so that the library needs no libcuda link.
+// sit elsewhere, so a new context id means a new lookup.
 constexpr int kNaMaxDevices = 64;
 struct NaSlot {
   unsigned long long ctx_id;
@@ -261,38 +259,12 @@ struct NaSlot {
 NaSlot g_na_slot[kNaMaxDevices] = {};
 std::mutex g_na_mutex;
 
-typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
-typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long*);
-
-// Id of the calling thread's current context, 0 if none or unknown.
-unsigned long long current_ctx_id() {
-  static CtxGetCurrentFn get_current = nullptr;
-  static CtxGetIdFn get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<CtxGetIdFn>(f);
-  });
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
-    return 0;
-  return id;
-}
-
 int na_scratch(int** out) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kNaMaxDevices) return VD_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_na_mutex);
   NaSlot& slot = g_na_slot[dev];
-  const unsigned long long id = current_ctx_id();
+  const unsigned long long id = vd::context_id();
   if (id != 0 && slot.addr && slot.ctx_id == id) {
     *out = slot.addr;
     return VD_OK;
@@ -302,7 +274,7 @@ int na_scratch(int** out) {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_na_scratch) != cudaSuccess || !p) return VD_ERR_CUDA;
   slot.addr = static_cast<int*>(p);
-  slot.ctx_id = current_ctx_id();  // 0 (unknown): looked up again on the next call
+  slot.ctx_id = vd::context_id();  // 0 (unknown): looked up again on the next call
   *out = slot.addr;
   return VD_OK;
 }
