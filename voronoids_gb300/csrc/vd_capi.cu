@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <new>
 #include <vector>
 
 #include "../../include/voronoids_gpu.h"
@@ -150,6 +151,7 @@ struct vd_tree {
     int64_t cap_slots = 0;
     double* q = nullptr;  // per query of a chunk
     int2* res = nullptr;
+    int* list = nullptr;  // queries of a chunk with large regions, then a counter
     int64_t cap_q = 0;
     int* out = nullptr;  // ranks of a chunk's regions
     int64_t cap_out = 0;
@@ -459,6 +461,7 @@ void release(vd_tree* t) {
   dfree(t->loc.tmp, t->stream);
   dfree(t->loc.q, t->stream);
   dfree(t->loc.res, t->stream);
+  dfree(t->loc.list, t->stream);
   dfree(t->loc.out, t->stream);
   dfree(t->d_counts, t->stream);
   dfree(t->T.lev_off, t->stream);
@@ -1877,60 +1880,101 @@ int vd_autotune_batch(vd_tree* t, const double* d_pts, const int64_t* offsets, i
   return rc;
 }
 
-// The m queries of S.q (numbers q0 ..) of vd_locate_points by the thread form,
-// whose per-query room grows with the largest region.
-static int locate_large(vd_tree* t, const vd::Launch& L, int nsimp, int64_t q0, int m, int64_t* offsets, int64_t* ids,
-                        int64_t cap, int64_t& total, bool& outside) {
-  const int dim = t->dim;
+// One chunk's regions on the host: region i is ids[at[i] .. at[i] + size[i]), size -1
+// outside the super simplex, -2 not known yet.
+namespace {
+struct Regions {
+  std::vector<int> size;
+  std::vector<int64_t> at;
+  std::vector<int2> res;
+  std::vector<int> ids;
+};
+
+// The first m queries of t->loc.q, or the n of t->loc.list (wide), in a warp form.
+// Ranks beyond `room` are not fetched: the caller has no place for them.
+int locate_warps(vd_tree* t, const vd::Launch& L, bool wide, int m, int n, bool want_ids, int64_t room, Regions& R) {
   vd_tree::LocateScratch& S = t->loc;
-  int *rank = nullptr, *flags = nullptr, *tmp = nullptr, *out = nullptr, *cnt = nullptr;
-  int cap_per = 256, rc = vd::E_OK;
-  std::vector<int> hc(m), ho;
-  if (dalloc(&flags, nsimp + 1, t->stream) || dalloc(&rank, nsimp + 1, t->stream) || dalloc(&tmp, vd::scan_scratch_ints(nsimp + 1), t->stream) ||
-      dalloc(&cnt, m, t->stream) || dalloc(&out, (size_t)m * cap_per, t->stream))
-    rc = vd::E_NOMEM;
-  if (!rc) vd::launch_live_rank(t->T, L, nsimp, flags, rank, tmp);
-  while (!rc) {
-    vd::launch_locate(t->T, L, dim, S.q, m, cap_per, rank, out, cnt);
-    cudaMemcpyAsync(hc.data(), cnt, sizeof(int) * m, cudaMemcpyDeviceToHost, t->stream);
-    rc = cuda_status(cudaStreamSynchronize(t->stream));
-    int need = 0;
-    for (int i = 0; i < m; ++i) need = std::max(need, hc[i]);
-    if (rc || need <= cap_per) break;
-    // a region larger than the per-query room (what did not fit was not
-    // searched on, so its true size is not known): once more with more
-    cap_per = std::max(need, 2 * cap_per);
-    dfree(out, t->stream);
-    if (dalloc(&out, (size_t)m * cap_per, t->stream)) rc = vd::E_NOMEM;
-  }
-  if (!rc) {
-    ho.resize((size_t)m * cap_per);
-    cudaMemcpyAsync(ho.data(), out, sizeof(int) * ho.size(), cudaMemcpyDeviceToHost, t->stream);
-    rc = cuda_status(cudaStreamSynchronize(t->stream));
-  }
-  for (int i = 0; i < m && !rc; ++i) {
-    const int c = std::max(hc[i], 0);
-    outside = outside || hc[i] < 0;
-    offsets[q0 + i + 1] = offsets[q0 + i] + c;
-    if (ids && total + c <= cap) {
-      int64_t* dst = ids + total;
-      for (int k = 0; k < c; ++k) dst[k] = ho[(size_t)i * cap_per + k];
-      std::sort(dst, dst + c);
+  int* total = S.list + S.cap_q;
+  const int64_t guess = wide ? 320LL * n + 1024 : (t->dim == 3 ? 40LL : 12LL) * n + 256;
+  int64_t want = want_ids ? std::max<int64_t>(S.cap_out, guess) : 0;
+  for (int attempt = 0;; ++attempt) {
+    if (want > S.cap_out) {
+      dfree(S.out, t->stream);
+      S.cap_out = 0;
+      if (want > 0x7fffffffLL || dalloc(&S.out, (size_t)want, t->stream)) return VD_ERR_NOMEM;
+      S.cap_out = want;
     }
-    total += c;
+    vd::launch_locate_warp(t->T, L, t->dim, wide, S.q, wide ? S.list : nullptr, n, S.rank, want_ids ? S.out : nullptr,
+                           (int)S.cap_out, S.res, total);
+    cudaMemcpyAsync(R.res.data(), S.res, sizeof(int2) * m, cudaMemcpyDeviceToHost, t->stream);
+    cudaMemcpyAsync(t->h_pair, total, sizeof(int), cudaMemcpyDeviceToHost, t->stream);
+    if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
+    if (!want_ids || t->h_pair[0] <= S.cap_out || attempt > 0) break;
+    want = t->h_pair[0];  // more ranks than the first guess: once more with enough room
   }
-  dfree(flags, t->stream);
-  dfree(rank, t->stream);
-  dfree(tmp, t->stream);
+  const int64_t base = (int64_t)R.ids.size();
+  const int k = t->h_pair[0];
+  if (want_ids && k > 0 && base + k <= room) {
+    R.ids.resize(base + k);
+    cudaMemcpyAsync(R.ids.data() + base, S.out, sizeof(int) * k, cudaMemcpyDeviceToHost, t->stream);
+    if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
+  }
+  for (int i = 0; i < m; ++i) {
+    if (wide && R.size[i] != -2) continue;
+    R.size[i] = R.res[i].x;
+    R.at[i] = base + R.res[i].y;
+  }
+  return VD_OK;
+}
+
+// The n queries of t->loc.list (their host copy: `list`) in the block form, as many at
+// a time as kLocateBytes of lists and bits allow, one at least.
+constexpr int64_t kLocateBytes = 256ll << 20;
+int locate_blocks(vd_tree* t, const vd::Launch& L, int nsimp, const std::vector<int>& list, bool want_ids, int64_t room,
+                  Regions& R) {
+  vd_tree::LocateScratch& S = t->loc;
+  const int n = (int)list.size();
+  const int64_t cap = std::max(nsimp, 1), words = ((int64_t)t->T.cap_simp + 31) / 32;
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>({n, 2LL * t->sms, kLocateBytes / (4 * (cap + words))}));
+  int *lists = nullptr, *cnt = nullptr;
+  unsigned* bits = nullptr;
+  int rc = VD_OK;
+  if (dalloc(&lists, (size_t)(G * cap), t->stream) || dalloc(&bits, (size_t)(G * words), t->stream) ||
+      dalloc(&cnt, G, t->stream))
+    rc = VD_ERR_NOMEM;
+  if (!rc) rc = cuda_status(cudaMemsetAsync(bits, 0, sizeof(unsigned) * G * words, t->stream));
+  try {
+    std::vector<int> hc(G);
+    for (int g0 = 0; g0 < n && !rc; g0 += G) {
+      const int g = std::min(G, n - g0);
+      vd::launch_locate_block(t->T, L, t->dim, S.q, S.list + g0, g, S.res, want_ids ? S.rank : nullptr, lists, cap, bits,
+                              words, cnt);
+      cudaMemcpyAsync(hc.data(), cnt, sizeof(int) * g, cudaMemcpyDeviceToHost, t->stream);
+      rc = cuda_status(cudaStreamSynchronize(t->stream));
+      for (int b = 0; b < g && !rc; ++b) {
+        const int i = list[g0 + b];
+        R.size[i] = hc[b];
+        R.at[i] = (int64_t)R.ids.size();
+        if (!want_ids || R.at[i] + hc[b] > room) continue;
+        R.ids.resize(R.at[i] + hc[b]);
+        cudaMemcpyAsync(R.ids.data() + R.at[i], lists + b * cap, sizeof(int) * hc[b], cudaMemcpyDeviceToHost, t->stream);
+        rc = cuda_status(cudaStreamSynchronize(t->stream));
+        std::sort(R.ids.begin() + R.at[i], R.ids.end());
+      }
+    }
+  } catch (const std::bad_alloc&) {
+    rc = VD_ERR_NOMEM;
+  }
+  dfree(lists, t->stream);
+  dfree(bits, t->stream);
   dfree(cnt, t->stream);
-  dfree(out, t->stream);
   return rc;
 }
 
-int vd_locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets, int64_t* ids, int64_t cap) {
-  if (ready(t) || !t->has_geometry || t->nsets != 1 || nq < 0 || (nq > 0 && !pts) || !offsets) return VD_ERR_ARG;
-  offsets[0] = 0;
-  if (nq == 0) return VD_OK;
+// vd_locate_points in chunks of queries.  Each chunk runs in the warp form; only
+// the queries whose regions outgrow its lists run in the wide one, and only those
+// that outgrow that in the block form.
+int locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets, int64_t* ids, int64_t cap) {
   int rc = sync_counters(t);
   if (rc) return rc;
   const int dim = t->dim;
@@ -1945,63 +1989,72 @@ int vd_locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets
     dfree(S.tmp, t->stream);
     S.cap_slots = 0;
     const int64_t c = nsimp + 1 + nsimp / 8;
-    if (dalloc(&S.flags, c, t->stream) || dalloc(&S.rank, c, t->stream) || dalloc(&S.tmp, vd::scan_scratch_ints(c), t->stream)) return VD_ERR_NOMEM;
+    if (dalloc(&S.flags, c, t->stream) || dalloc(&S.rank, c, t->stream) ||
+        dalloc(&S.tmp, vd::scan_scratch_ints(c), t->stream))
+      return VD_ERR_NOMEM;
     S.cap_slots = c;
   }
   if (chunk > S.cap_q) {
     dfree(S.q, t->stream);
     dfree(S.res, t->stream);
+    dfree(S.list, t->stream);
     S.cap_q = 0;
-    if (dalloc(&S.q, (size_t)(chunk * dim), t->stream) || dalloc(&S.res, chunk + 1, t->stream)) return VD_ERR_NOMEM;
+    if (dalloc(&S.q, (size_t)(chunk * dim), t->stream) || dalloc(&S.res, chunk, t->stream) ||
+        dalloc(&S.list, chunk + 1, t->stream))
+      return VD_ERR_NOMEM;
     S.cap_q = chunk;
   }
   if (ids) vd::launch_live_rank(t->T, L, nsimp, S.flags, S.rank, S.tmp);
-  std::vector<int2> hr(chunk + 1);
-  std::vector<int> ho;
+  Regions R;
+  R.size.resize(chunk);
+  R.at.resize(chunk);
+  R.res.resize(chunk);
+  std::vector<int> big;
   bool outside = false;
   int64_t total = 0;
-  for (int64_t q0 = 0; q0 < nq && !rc; q0 += chunk) {
+  auto collect = [&](int m) {  // queries whose region outgrew the lists
+    big.clear();
+    for (int i = 0; i < m; ++i)
+      if (R.size[i] == -2) big.push_back(i);
+    if (!big.empty())
+      cudaMemcpyAsync(S.list, big.data(), sizeof(int) * big.size(), cudaMemcpyHostToDevice, t->stream);
+    return !big.empty();
+  };
+  for (int64_t q0 = 0; q0 < nq; q0 += chunk) {
     const int m = (int)std::min<int64_t>(chunk, nq - q0);
+    const int64_t room = cap - total;
     cudaMemcpyAsync(S.q, pts + q0 * dim, sizeof(double) * m * dim, cudaMemcpyHostToDevice, t->stream);
-    int64_t want = ids ? std::max<int64_t>(S.cap_out, (dim == 3 ? 40LL : 12LL) * m + 256) : 0;
-    bool large = false;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      if (want > S.cap_out) {
-        dfree(S.out, t->stream);
-        S.cap_out = 0;
-        if (want > 0x7fffffffLL || dalloc(&S.out, (size_t)want, t->stream)) return VD_ERR_NOMEM;
-        S.cap_out = want;
-      }
-      vd::launch_locate_warp(t->T, L, dim, S.q, m, S.rank, ids ? S.out : nullptr, (int)S.cap_out, S.res);
-      cudaMemcpyAsync(hr.data(), S.res, sizeof(int2) * (m + 1), cudaMemcpyDeviceToHost, t->stream);
-      if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
-      if (!ids || hr[m].x <= S.cap_out) break;
-      want = hr[m].x;  // more ranks than the first guess: once more with enough room
-    }
-    for (int i = 0; i < m; ++i) large = large || hr[i].x == -2;
-    if (large) {
-      rc = locate_large(t, L, nsimp, q0, m, offsets, ids, cap, total, outside);
-      continue;
-    }
-    const int k = hr[m].x;
-    if (ids && k > 0) {
-      ho.resize(k);
-      cudaMemcpyAsync(ho.data(), S.out, sizeof(int) * k, cudaMemcpyDeviceToHost, t->stream);
-      if (cudaStreamSynchronize(t->stream) != cudaSuccess) return VD_ERR_CUDA;
-    }
+    R.ids.clear();
+    rc = locate_warps(t, L, false, m, m, ids != nullptr, room, R);
+    if (!rc && collect(m)) rc = locate_warps(t, L, true, m, (int)big.size(), ids != nullptr, room, R);
+    if (!rc && !big.empty() && collect(m)) rc = locate_blocks(t, L, nsimp, big, ids != nullptr, room, R);
+    if (rc) return rc;
     for (int i = 0; i < m; ++i) {
-      const int c = std::max(hr[i].x, 0);
-      outside = outside || hr[i].x < 0;
+      const int c = std::max(R.size[i], 0);
+      outside = outside || R.size[i] < 0;
       offsets[q0 + i + 1] = offsets[q0 + i] + c;
-      if (ids && total + c <= cap) std::copy(ho.begin() + hr[i].y, ho.begin() + hr[i].y + c, ids + total);
+      if (ids && total + c <= cap && R.at[i] + c <= (int64_t)R.ids.size())
+        std::copy(R.ids.begin() + R.at[i], R.ids.begin() + R.at[i] + c, ids + total);
       total += c;
     }
   }
-  if (!rc) rc = sync_counters(t);
+  rc = sync_counters(t);
   if (rc) return rc;
   if (t->hctr->err) return t->hctr->err;
   if (ids && total > cap) return VD_ERR_ARG;
   return outside ? VD_ERR_OUTSIDE : VD_OK;
+}
+}  // namespace
+
+int vd_locate_points(vd_tree* t, const double* pts, int64_t nq, int64_t* offsets, int64_t* ids, int64_t cap) {
+  if (ready(t) || !t->has_geometry || t->nsets != 1 || nq < 0 || (nq > 0 && !pts) || !offsets) return VD_ERR_ARG;
+  offsets[0] = 0;
+  if (nq == 0) return VD_OK;
+  try {
+    return locate_points(t, pts, nq, offsets, ids, cap);
+  } catch (const std::bad_alloc&) {
+    return VD_ERR_NOMEM;
+  }
 }
 
 int vd_circumspheres(vd_tree* t, double* centers, double* radii, int64_t cap, int64_t* n) {

@@ -368,20 +368,23 @@ struct EdgeScratch {
 int64_t scan_scratch_ints(int64_t n);
 // out[i] = sum(in[0..i)) for i < n, out[n] = total; tmp: scan_scratch_ints(n).
 void scan_ints(const int* in, int* out, int64_t n, int* tmp, cudaStream_t st);
-// Conflict regions of nq query points (vd_locate.cu): slots of query i in
-// out[i * cap_per ..] numbered by rank[], count in counts[i] (-1: outside
-// the super simplex; above cap_per: truncated).  rank[s] = position of live
-// slot s among the
-// live slots (nsimp + 1 entries, tmp: scan_scratch_ints(nsimp)).
-void launch_locate(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, int cap_per,
-                   const int* rank, int* out, int* counts);
+// rank[s] = position of live slot s among the live slots (nsimp + 1 entries,
+// tmp: scan_scratch_ints(nsimp)).
 void launch_live_rank(const DevTree& T, const Launch& L, int nsimp, int* flags, int* rank, int* tmp);
-// The same, a warp per query: res[i] = (count, first) with the sorted ranks of
-// query i at out[first ..], count -1 outside the super simplex, -2 too large
-// for a warp (launch_locate does it); res[nq].x = ranks in all, which may
-// exceed cap_out.  out null: counts only.
-void launch_locate_warp(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, const int* rank, int* out,
-                        int cap_out, int2* res);
+// Conflict regions of n query points (vd_locate.cu): those of `list`, or 0 .. n - 1
+// without one.  A warp per query: res[i] = (count, first) with the sorted ranks of
+// query i at out[first ..], count -1 outside the super simplex, -2 too large for
+// the form's lists (`first` is a simplex of the region); *total = ranks in all,
+// which may exceed cap_out.  out null: counts only.
+void launch_locate_warp(const DevTree& T, const Launch& L, int dim, bool wide, const double* d_q, const int* list, int n,
+                        const int* rank, int* out, int cap_out, int2* res, int* total);
+// The same for regions of any size, a block per query: query list[b] starts at
+// res[list[b]].y; its region (ranks where `rank` is given) in lists[b * cap ..] in no
+// order, its size in cnt[b].  cap: slots of the tree; bits: n * words words, zero on
+// entry and left zero, a bit per slot below T.cap_simp.
+void launch_locate_block(const DevTree& T, const Launch& L, int dim, const double* d_q, const int* list, int n,
+                         const int2* res, const int* rank, int* lists, int64_t cap, unsigned* bits, int64_t words,
+                         int* cnt);
 // Circumcentre (3 doubles, z = 0 in 2D) and radius of each live simplex,
 // written at its rank.
 void launch_circum(const DevTree& T, const Launch& L, int dim, int nsimp, const int* rank, double* centers,

@@ -4,8 +4,9 @@
 //
 // A visibility walk from the finest location hint of the set towards the
 // simplex that contains the point, then a breadth-first search over face
-// neighbours with the exact conflict test: a warp per query, or a thread per
-// query where a region outgrows the warp's lists.  The query takes the role of
+// neighbours with the exact conflict test: a warp per query with lists in
+// shared memory, small ones and then large ones, and a block per query with
+// lists as long as the tree for what outgrows both.  The query takes the role of
 // the newest vertex (largest id), so a point exactly on a circumsphere is
 // outside: the reference's strict `dist < r`.  The conflict region is
 // connected, so the search finds all of it.
@@ -62,74 +63,92 @@ __device__ __forceinline__ bool hset_add(int* hk, int key) {
   return false;
 }
 
+// 1 if the query p (record fp) is in conflict with simplex s (vertices v), -1 if
+// not; with `sphere` alone 0 where the stored sphere (3D) cannot decide.
+template <int D>
+__device__ __forceinline__ int query_side(const DevTree& T, int s, const int4& v, const vdp::VPt& p, const vdp::FPt& fp,
+                                          bool sphere, vdp::Tally& tl, int& perr) {
+  constexpr int NV = D + 1;
+  if (D == 3) {
+    const float4 c = *reinterpret_cast<const float4*>(T.sph + s);
+    const int side = vdp::sphere_side<D>(vdp::Sph{c.x, c.y, c.z, c.w}, fp);
+    if (side != 0) return side;
+  }
+  if (sphere) return 0;
+  vdp::FPt fv[NV];
+  int key[NV];
+  for (int j = 0; j < NV; ++j) {
+    key[j] = g4(v, j);
+    fv[j] = T.ptf[key[j]];
+  }
+  auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
+    for (int j = 0; j < NV; ++j) v64[j] = T.pts[key[j]];
+    p64 = p;
+  };
+  const int qkey = 0x7fffffff;  // newer than every vertex
+  return vdp::in_conflict_hl<D>(fv, key, fp, qkey, tl, perr, load64) ? 1 : -1;
+}
+
+template <int D>
+__device__ __forceinline__ void load_query(const double* q, int i, vdp::VPt& p, vdp::FPt& fp) {
+  p = vdp::VPt{q[(long long)i * D], q[(long long)i * D + 1], D == 3 ? q[(long long)i * D + 2] : 0.0, 0.0};
+  fp = vdp::split_point(p.x, p.y, p.z);
+}
+
 // Warp form: a warp per query, region lists in shared memory.  The walk stops
 // at the first simplex whose stored sphere (3D) certainly holds the point: the
 // conflict region is connected, so any of its simplices will do to start from.
 // The region is searched in waves of 32 (simplex, face) items, as in the
 // insertion rounds.  Bound by the chain of dependent gathers of one query
-// (walk, then about six waves), with every query of a call in flight; the
-// thread form below did a region's 50 tests one after another (4,096 queries in
-// a 100,000-point tree: 1.2 ms a call, this form about 0.1 ms).
+// (walk, then about six waves), with every query of a call in flight: the
+// kernel takes about 0.1 ms for 4,096 queries in a 100,000-point tree.
 //
-// res[i] = (count, first) of query i: count -1 outside the super simplex, -2
-// when the region outgrew the lists (the caller then uses the thread form); its
-// sorted ranks are out[first ..].  res[nq].x counts the ranks of all queries,
-// which may exceed cap_out; with out null only the counts are made.
-constexpr int kLocWarps = 4;
-template <int D>
+// Queries are 0 .. n - 1, or list[0 .. n) where a list is given.  res[i] =
+// (count, first) of query i: count -1 outside the super simplex, -2 when the
+// region outgrew the lists (`first` is then a simplex of the region); its
+// sorted ranks are out[first ..].  *total counts the ranks of all queries, which
+// may exceed cap_out; with out null only the counts are made.
+//
+// WIDE: the lists are 192 simplices in 3D and 64 in 2D, with 16 warps on an
+// SM; the wide form, for the queries that outgrow these, has 1,024 and six warps.
+template <int D, bool WIDE>
 struct LocWarp {
-  static constexpr int CAP = D == 3 ? 192 : 64, HS = D == 3 ? 512 : 128;
+  static constexpr int WARPS = WIDE ? 1 : 4, BLOCKS = WIDE ? 6 : 4;
+  static constexpr int CAP = WIDE ? 1024 : (D == 3 ? 192 : 64), HS = WIDE ? 4096 : (D == 3 ? 512 : 128);
   int4 cn[CAP];
   int hk[HS];  // id set of the region, then its ranks while they are sorted
   int cav[CAP];
 };
 
-template <int D>
-__global__ void __launch_bounds__(32 * kLocWarps, 4) k_locate_warp(DevTree T, const double* q, int nq, const int* rank,
-                                                                  int* out, int cap_out, int2* res) {
-  constexpr int NV = D + 1, CAP = LocWarp<D>::CAP, HS = LocWarp<D>::HS;
+template <int D, bool WIDE>
+__global__ void __launch_bounds__(32 * LocWarp<D, WIDE>::WARPS, LocWarp<D, WIDE>::BLOCKS)
+    k_locate_warp(DevTree T, const double* q, const int* list, int n_list, const int* rank, int* out, int cap_out,
+                  int2* res, int* total) {
+  using Warp = LocWarp<D, WIDE>;
+  constexpr int NV = D + 1, CAP = Warp::CAP, HS = Warp::HS;
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ LocWarp<D> sm[kLocWarps];
-  LocWarp<D>& W = sm[threadIdx.x >> 5];
+  __shared__ Warp sm[Warp::WARPS];
+  Warp& W = sm[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  const int qkey = 0x7fffffff;  // newer than every vertex
   vdp::Tally tl = {0, 0, 0, 0};
   int perr = 0;
   const SetGeo& g = T.sets[0];
-  for (int i = blockIdx.x * kLocWarps + (threadIdx.x >> 5); i < nq; i += gridDim.x * kLocWarps) {
-    const vdp::VPt p{q[(long long)i * D], q[(long long)i * D + 1], D == 3 ? q[(long long)i * D + 2] : 0.0, 0.0};
-    const vdp::FPt fp = vdp::split_point(p.x, p.y, p.z);
-    auto verts = [&](const int4& v, vdp::FPt* fv) {
-      for (int j = 0; j < NV; ++j) fv[j] = T.ptf[g4(v, j)];
-    };
+  for (int j0 = blockIdx.x * Warp::WARPS + (threadIdx.x >> 5); j0 < n_list; j0 += gridDim.x * Warp::WARPS) {
+    const int i = list ? list[j0] : j0;
+    vdp::VPt p;
+    vdp::FPt fp;
+    load_query<D>(q, i, p, fp);
     auto exit_of = [&](const int4& v) {
       vdp::FPt fv[NV];
-      verts(v, fv);
+      for (int j = 0; j < NV; ++j) fv[j] = T.ptf[g4(v, j)];
       auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
         for (int j = 0; j < NV; ++j) v64[j] = T.pts[g4(v, j)];
         p64 = p;
       };
       return vdp::exit_face_hl<D>(fv, fp, (1u << NV) - 1, tl, perr, load64);
     };
-    // 1 in conflict, -1 not; with `sphere` alone 0 where it cannot decide
-    auto conflict = [&](int s, const int4& v, bool sphere) {
-      if (D == 3) {
-        const float4 c = *reinterpret_cast<const float4*>(T.sph + s);
-        const int side = vdp::sphere_side<D>(vdp::Sph{c.x, c.y, c.z, c.w}, fp);
-        if (side != 0) return side;
-      }
-      if (sphere) return 0;
-      vdp::FPt fv[NV];
-      int key[NV];
-      verts(v, fv);
-      for (int j = 0; j < NV; ++j) key[j] = g4(v, j);
-      auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
-        for (int j = 0; j < NV; ++j) v64[j] = T.pts[key[j]];
-        p64 = p;
-      };
-      return vdp::in_conflict_hl<D>(fv, key, fp, qkey, tl, perr, load64) ? 1 : -1;
-    };
+    auto conflict = [&](int s, const int4& v, bool sphere) { return query_side<D>(T, s, v, p, fp, sphere, tl, perr); };
     int cur = -1;
     for (int l = g.hint_levels; l >= 0 && cur < 0; --l) cur = T.hint[hint_cell<D>(g, p, l)];
     if (cur < 0 || bad_simp(T, cur)) cur = g.root;
@@ -206,8 +225,9 @@ __global__ void __launch_bounds__(32 * kLocWarps, 4) k_locate_warp(DevTree T, co
     int first = 0;
     if (n > CAP) {
       n = -2;
+      first = cur;
     } else if (n > 0 && out) {
-      if (lane == 0) first = atomicAdd(&res[nq].x, n);
+      if (lane == 0) first = atomicAdd(total, n);
       first = __shfl_sync(FULL, first, 0);
       // the ranks (numbering of the simplex export), sorted
       int P = 32;
@@ -231,102 +251,75 @@ __global__ void __launch_bounds__(32 * kLocWarps, 4) k_locate_warp(DevTree T, co
         for (int k = lane; k < n; k += 32) out[first + k] = W.hk[k];
       __syncwarp();
     } else if (n > 0 && lane == 0) {
-      atomicAdd(&res[nq].x, n);
+      atomicAdd(total, n);
     }
     if (lane == 0) res[i] = make_int2(n, first);
   }
   if (perr) set_error(T.ctr, E_PRECISION);
 }
 
+// Block form: a block per query list[b], which starts at res[list[b]].y (a simplex of
+// its region).  The region's simplices are a set of bits over the slots and a
+// list, both of the block's own and as long as the tree, so no region is too
+// large; the bits are zero on entry and on return.  Waves take every (simplex,
+// face) item found so far, kLocThreads at a time.  lists[b * cap ..] receives the
+// region as ranks (rank given) in no order, cnt[b] its size.
+constexpr int kLocThreads = 256;
 template <int D>
-__global__ void k_locate(DevTree T, const double* q, int nq, int cap_per, const int* rank, int* out, int* counts) {
+__global__ void __launch_bounds__(kLocThreads) k_locate_block(DevTree T, const double* q, const int* list, const int2* res,
+                                                              const int* rank, int* lists, long long cap, unsigned* bits,
+                                                              long long words, int* cnt) {
   constexpr int NV = D + 1;
-  const int qkey = 0x7fffffff;  // newer than every vertex
+  __shared__ int s_n;
+  const int b = blockIdx.x, i = list[b];
+  int* L = lists + b * cap;
+  unsigned* B = bits + b * words;
   vdp::Tally tl = {0, 0, 0, 0};
   int perr = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
-    const vdp::VPt p{q[(long long)i * D], q[(long long)i * D + 1], D == 3 ? q[(long long)i * D + 2] : 0.0, 0.0};
-    const vdp::FPt fp = vdp::split_point(p.x, p.y, p.z);
-    const SetGeo& g = T.sets[0];
-    int cur = -1;
-    for (int l = g.hint_levels; l >= 0 && cur < 0; --l) cur = T.hint[hint_cell<D>(g, p, l)];
-    if (cur < 0 || bad_simp(T, cur)) cur = g.root;
-    int4 v, nn;
-    load_simp(T, cur, v, nn);
-    for (int k = 0; k < 64 && v.x < 0 && nn.x >= 0; ++k) {  // dead slot: into its star
-      cur = nn.x >> 2;
-      if (bad_simp(T, cur)) break;
-      load_simp(T, cur, v, nn);
-    }
-    int* o = out + (long long)i * cap_per;
-    if (v.x < 0 || bad_simp(T, cur)) {
+  vdp::VPt p;
+  vdp::FPt fp;
+  load_query<D>(q, i, p, fp);
+  const int start = res[i].y;
+  if (bad_simp(T, start)) {
+    if (threadIdx.x == 0) {
       set_error(T.ctr, E_INTERNAL);
-      counts[i] = 0;
-      continue;
+      cnt[b] = 0;
     }
-    // visibility walk
-    bool outside = false;
-    for (int step = 0; step < (1 << 16); ++step) {
-      vdp::FPt fv[NV];
-      for (int j = 0; j < NV; ++j) fv[j] = T.ptf[g4(v, j)];
-      auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
-        for (int j = 0; j < NV; ++j) v64[j] = T.pts[g4(v, j)];
-        p64 = p;
-      };
-      const int f = vdp::exit_face_hl<D>(fv, fp, (1u << NV) - 1, tl, perr, load64);
-      if (f < 0) break;
-      const int code = g4(nn, f);
-      if (code < 0 || bad_simp(T, code >> 2)) {
-        outside = code < 0;
-        break;
-      }
-      cur = code >> 2;
-      load_simp(T, cur, v, nn);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    s_n = 1;
+    L[0] = start;
+    atomicOr(B + (start >> 5), 1u << (start & 31));
+  }
+  for (long long head = 0;;) {
+    __syncthreads();
+    const long long avail = (long long)s_n * NV;
+    __syncthreads();
+    if (head >= avail) break;
+    for (long long it = head + threadIdx.x; it < avail; it += kLocThreads) {
+      const int k = (int)(it / NV), f = (int)(it - (long long)k * NV);
+      const int code = reinterpret_cast<const int*>(T.simp + L[k])[4 + f];
+      const int nb = code >> 2;
+      if (code < 0 || bad_simp(T, nb) || (__ldcg(B + (nb >> 5)) >> (nb & 31) & 1u)) continue;
+      int4 v, n;
+      load_simp(T, nb, v, n);
+      if (query_side<D>(T, nb, v, p, fp, false, tl, perr) < 0) continue;
+      if (atomicOr(B + (nb >> 5), 1u << (nb & 31)) >> (nb & 31) & 1u) continue;  // another thread has it
+      const int at = atomicAdd(&s_n, 1);
+      if (at < cap) L[at] = nb;
     }
-    if (outside) {
-      counts[i] = -1;
-      continue;
-    }
-    // breadth-first search of the conflict region (the containing simplex
-    // is in it unless the point is one of its vertices)
-    int cnt = 0;
-    auto conflict = [&](int s, const int4& sv) {
-      vdp::FPt fv[NV];
-      int key[NV];
-      for (int j = 0; j < NV; ++j) {
-        key[j] = g4(sv, j);
-        fv[j] = T.ptf[key[j]];
-      }
-      auto load64 = [&](vdp::VPt* v64, vdp::VPt& p64) {
-        for (int j = 0; j < NV; ++j) v64[j] = T.pts[key[j]];
-        p64 = p;
-      };
-      return vdp::in_conflict_hl<D>(fv, key, fp, qkey, tl, perr, load64);
-    };
-    if (conflict(cur, v)) {
-      if (cap_per > 0) o[0] = cur;
-      cnt = 1;
-    }
-    for (int h = 0; h < cnt && h < cap_per; ++h) {
-      int4 cv, cn;
-      load_simp(T, o[h], cv, cn);
-      for (int f = 0; f < NV; ++f) {
-        const int code = g4(cn, f);
-        if (code < 0) continue;
-        const int nb = code >> 2;
-        if (bad_simp(T, nb)) continue;
-        bool seen = false;
-        for (int k = 0; k < cnt && k < cap_per && !seen; ++k) seen = o[k] == nb;
-        if (seen) continue;
-        int4 bv, bn;
-        load_simp(T, nb, bv, bn);
-        if (!conflict(nb, bv)) continue;
-        if (cnt < cap_per) o[cnt] = nb;
-        ++cnt;
-      }
-    }
-    for (int k = 0; k < cnt && k < cap_per; ++k) o[k] = rank[o[k]];  // numbering of the simplex export
-    counts[i] = cnt;
+    head = avail;
+  }
+  const int n = (int)min((long long)s_n, cap);  // a region has at most the tree's simplices
+  if (threadIdx.x == 0) {
+    if (s_n > cap) set_error(T.ctr, E_INTERNAL);
+    cnt[b] = n;
+  }
+  for (int k = threadIdx.x; k < n; k += kLocThreads) {
+    const int s = L[k];
+    B[s >> 5] = 0u;  // every set bit of the word belongs to this region
+    if (rank) L[k] = rank[s];
   }
   if (perr) set_error(T.ctr, E_PRECISION);
 }
@@ -388,25 +381,37 @@ void launch_circum(const DevTree& T, const Launch& L, int dim, int nsimp, const 
     k_circum<2><<<L.blocks, 256, 0, L.stream>>>(T, nsimp, rank, centers, radii);
 }
 
-void launch_locate(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, int cap_per,
-                   const int* rank, int* out, int* counts) {
+namespace {
+template <int D, bool WIDE>
+void locate_warp(const DevTree& T, const Launch& L, const double* d_q, const int* list, int n, const int* rank, int* out,
+                 int cap_out, int2* res, int* total) {
+  constexpr int W = LocWarp<D, WIDE>::WARPS;
+  const int blocks = std::max(1, std::min((n + W - 1) / W, L.blocks));
+  k_locate_warp<D, WIDE><<<blocks, 32 * W, 0, L.stream>>>(T, d_q, list, n, rank, out, cap_out, res, total);
+}
+}  // namespace
+
+void launch_locate_warp(const DevTree& T, const Launch& L, int dim, bool wide, const double* d_q, const int* list, int n,
+                        const int* rank, int* out, int cap_out, int2* res, int* total) {
   note_launches(1);
-  const int blocks = std::max(1, std::min((nq + 127) / 128, L.blocks * 2));
-  if (dim == 3)
-    k_locate<3><<<blocks, 128, 0, L.stream>>>(T, d_q, nq, cap_per, rank, out, counts);
-  else
-    k_locate<2><<<blocks, 128, 0, L.stream>>>(T, d_q, nq, cap_per, rank, out, counts);
+  cudaMemsetAsync(total, 0, sizeof(int), L.stream);
+  if (dim == 3) {
+    if (wide) locate_warp<3, true>(T, L, d_q, list, n, rank, out, cap_out, res, total);
+    else locate_warp<3, false>(T, L, d_q, list, n, rank, out, cap_out, res, total);
+  } else {
+    if (wide) locate_warp<2, true>(T, L, d_q, list, n, rank, out, cap_out, res, total);
+    else locate_warp<2, false>(T, L, d_q, list, n, rank, out, cap_out, res, total);
+  }
 }
 
-void launch_locate_warp(const DevTree& T, const Launch& L, int dim, const double* d_q, int nq, const int* rank, int* out,
-                        int cap_out, int2* res) {
+void launch_locate_block(const DevTree& T, const Launch& L, int dim, const double* d_q, const int* list, int n,
+                         const int2* res, const int* rank, int* lists, int64_t cap, unsigned* bits, int64_t words,
+                         int* cnt) {
   note_launches(1);
-  cudaMemsetAsync(res + nq, 0, sizeof(int2), L.stream);
-  const int blocks = std::max(1, std::min((nq + kLocWarps - 1) / kLocWarps, L.blocks));
   if (dim == 3)
-    k_locate_warp<3><<<blocks, 32 * kLocWarps, 0, L.stream>>>(T, d_q, nq, rank, out, cap_out, res);
+    k_locate_block<3><<<n, kLocThreads, 0, L.stream>>>(T, d_q, list, res, rank, lists, cap, bits, words, cnt);
   else
-    k_locate_warp<2><<<blocks, 32 * kLocWarps, 0, L.stream>>>(T, d_q, nq, rank, out, cap_out, res);
+    k_locate_block<2><<<n, kLocThreads, 0, L.stream>>>(T, d_q, list, res, rank, lists, cap, bits, words, cnt);
 }
 
 void launch_live_rank(const DevTree& T, const Launch& L, int nsimp, int* flags, int* rank, int* tmp) {
