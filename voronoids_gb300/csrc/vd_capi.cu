@@ -543,6 +543,9 @@ int alloc_tree(vd_tree* t, int dim, void* stream) {
       dalloc(&t->d_misc, 16, t->stream) || dalloc(&t->d_counts, 2 * vd::kMaxLevels, t->stream) ||
       dalloc(&t->T.lev_off, vd::kMaxLevels + 1, t->stream))
     return vd::E_NOMEM;
+  // an empty tree can be asked for its counts, and the pool's memory holds an
+  // earlier tree's
+  if (cudaMemsetAsync(t->T.ctr, 0, sizeof(Counters), t->stream) != cudaSuccess) return vd::E_CUDA;
   t->T.cap_wchunk = t->sms * kChunkWarpsPerSm;
   if (dalloc(&t->T.wchunk, t->T.cap_wchunk, t->stream)) return vd::E_NOMEM;
   t->ncells = vd::hint_cells(dim, single_hint_levels(dim));
@@ -1135,6 +1138,11 @@ int compute_edges(vd_tree* t, uint2* out = nullptr, int64_t cap = 0, int64_t* m 
   }
   int rc = sync_counters(t);
   if (rc) return rc;
+  if (!t->has_geometry) {  // vd_tree_create: no points and no scratch yet
+    t->nedges = 0;
+    if (m) *m = 0;
+    return vd::E_OK;
+  }
   const int64_t n_in = t->nverts - t->ns;
   const int64_t nsimp = t->hctr->nsimp;
   if ((t->dim == 3 ? 6 : 3) * nsimp > 0x7fffff00LL) return vd::E_NOMEM;
