@@ -83,6 +83,11 @@ vd_tree* vd_tree_new(int dim, const double* pts, int64_t n, int* status);
 /* Same, with all device work on the caller's CUDA stream (cudaStream_t). */
 vd_tree* vd_tree_new_on_stream(int dim, const double* pts, int64_t n, void* stream, int* status);
 void vd_tree_free(vd_tree* t);
+/* Device memory of freed trees serves the next ones: up to 512 MB per device
+ * (and 16 pinned host blocks of 8 KB) stay with the library, the rest goes back
+ * when a tree is freed.  This gives all of it back, on the calling thread's
+ * device; it waits for the device.  Live trees keep their memory. */
+int vd_trim_memory(void);
 /* `new` from points already in device memory (n * dim doubles).  The super
  * simplex is bit-identical to the host path's. */
 vd_tree* vd_tree_new_device(int dim, const double* d_pts, int64_t n, void* stream, int* status);

@@ -48,7 +48,8 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* q) {
 }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) { memset(v, 0, 8); return cudaSuccess; }
-cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t mp, size_t) { if (!alive(pools, mp)) ++faults; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t mp, cudaStream_t) {
   if (!alive(pools, mp) || pools[mp] != ctx_of[dev]) { ++faults; return cudaErrorInvalidValue; }
   *p = malloc(n);
@@ -81,6 +82,7 @@ void* take(void) { return vd::pinned_alloc(&owner); }
 unsigned long long taken_owner(void) { return owner; }
 void give(void* p, unsigned long long c) { vd::pinned_free(p, c); }
 int usable(void* p) { return alive(pinned, p) && pinned[p] == ctx_of[dev]; }
+int trim(void) { return vd::pool_trim(); }
 void* array(void) { return vd::pool_alloc(64, nullptr); }
 void array_free(void* p) { vd::pool_free(p, nullptr); }
 }
@@ -149,3 +151,12 @@ def test_a_block_given_back_after_its_context_ended_is_not_handed_out(mem):
     mem.give(p, c)
     assert mem.usable(mem.take())
     assert mem.fault_count() == 0
+
+
+def test_a_trim_after_a_reset_touches_nothing_dead(mem):
+    p, c = mem.take(), mem.taken_owner()
+    mem.give(p, c)
+    assert mem.array() and mem.trim() == 0
+    assert mem.usable(mem.take()) and mem.made_count() == 2  # the kept block was given back
+    mem.reset()
+    assert mem.trim() == 0 and mem.array() and mem.fault_count() == 0

@@ -243,6 +243,8 @@ unsigned long long context_id();
 // takes null, and a stream that is gone.
 void* pool_alloc(size_t bytes, cudaStream_t st);
 void pool_free(void* p, cudaStream_t st);
+// What the current context's pool and pinned list keep, given back.
+int pool_trim();
 // Pinned host blocks of kPinnedBytes; `context` is the context that a block
 // belongs to.
 constexpr size_t kPinnedBytes = 8192;

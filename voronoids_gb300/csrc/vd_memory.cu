@@ -5,8 +5,9 @@
 // from a stream-ordered pool: what one tree gives back the next one takes, from
 // any thread and on any stream (the pool orders a block's reuse after its free).
 // Up to kKeepBytes of free memory stay with the pool; the rest goes back to the
-// device at the next synchronisation, and all of it when an allocation fails.
-// Pinned blocks are kept in a short list.
+// device at the next synchronisation (a tree that is freed makes one), and all of
+// it when an allocation fails or the caller asks (vd_trim_memory).  Pinned blocks
+// are kept in a short list.
 //
 // Pool and list belong to a CUDA context and end with it (cudaDeviceReset, or a
 // device's primary context given up by all of its users), so they are looked up
@@ -134,6 +135,15 @@ void pool_free(void* p, cudaStream_t st) {
   if (pool() && cudaFreeAsync(p, st) == cudaSuccess) return;
   cudaGetLastError();
   cudaFree(p);  // waits for the device
+}
+
+int pool_trim() {
+  std::lock_guard<std::mutex> lock(g_mu);
+  ContextMemory* e = current_entry();
+  if (!e) return E_OK;  // nothing is kept without a context
+  if (cudaDeviceSynchronize() != cudaSuccess) return E_CUDA;  // frees still in their streams
+  while (e->npinned > 0) cudaFreeHost(e->pinned[--e->npinned]);
+  return e->pool && cudaMemPoolTrimTo(e->pool, 0) != cudaSuccess ? E_CUDA : E_OK;
 }
 
 void* pinned_alloc(unsigned long long* context) {

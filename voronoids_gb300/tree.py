@@ -379,6 +379,11 @@ class DelaunayTree:
         return {k: getattr(s, k) for k, _ in s._fields_}
 
 
+def trim_memory():
+    """Give the device memory that the library keeps for later trees (at most 512 MB) back now."""
+    _check(_native.load().vd_trim_memory(), "trim_memory")
+
+
 def check_triangulation(points, verts, nbrs):
     """``check_delaunay`` on a caller's triangulation (``vd_check_triangulation``).
 
