@@ -313,7 +313,7 @@ class DelaunayTree:
                                    n.value, ctypes.byref(n)), "duplicates")
         return out
 
-    def set_schedule(self, first_prefix=64, growth=1.25, ratio=0.12):
+    def set_schedule(self, first_prefix=64, growth=1.4, ratio=0.12):
         _check(_native.load().vd_set_schedule(self._h, int(first_prefix), float(growth), float(ratio)),
                "set_schedule")
 
