@@ -2271,6 +2271,7 @@ __global__ void __launch_bounds__(32) k_insert_one(DevTree T, double x, double y
         }
         load_simplex(T, cur, v, nn);
       }
+      if (s_status == 0 && v.x < 0) s_status = E_INTERNAL;  // still dead: its stored sphere is an old simplex's
       // the walk may end before the simplex that contains the point, at one
       // whose stored sphere certainly holds it (3D): the region is connected,
       // and such a point equals no vertex, since no vertex lies inside a sphere
