@@ -271,6 +271,11 @@ const char* vd_profile_name(int i);
 int vd_set_trace(vd_tree* t, int on);
 /* Kernels launched by this library in this process so far. */
 int64_t vd_kernel_launches(void);
+/* Paths that a tree's work took, 3 entries: points of the current triangulation
+ * that were inserted under locks at the end of a call instead of in rounds;
+ * rounds captured as CUDA graphs since the tree was made; rounds replayed from
+ * graphs that an earlier call captured. */
+int vd_path_counts(vd_tree* t, int64_t* out);
 int vd_trace(vd_tree* t, int64_t* rows, int64_t cap, int64_t* n);
 
 /* voronoids.delaunay(points) (src/lib.rs:104-125) in one call: new + insert

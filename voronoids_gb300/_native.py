@@ -29,7 +29,7 @@ EXPORTS = [
     "vd_batch_delaunay", "vd_batch_delaunay_device", "vd_num_sets", "vd_tree_create",
     "vd_set_launch", "vd_autotune_batch", "vd_locate_points", "vd_set_adjacent", "vd_circumspheres", "vd_set_small_rounds", "vd_set_early_phase", "vd_set_exact_tier", "vd_set_first_block",
     "vd_server_new", "vd_server_submit", "vd_server_poll", "vd_server_result", "vd_server_stats", "vd_server_free",
-    "vd_check_triangulation", "vd_voronoi_edges", "vd_voronoi_cells", "vd_trim_memory",
+    "vd_check_triangulation", "vd_voronoi_edges", "vd_voronoi_cells", "vd_trim_memory", "vd_path_counts",
 ]
 
 
@@ -117,6 +117,7 @@ def load(path=LIB_PATH):
         "vd_trace": ([vp, i64p, i64, i64p], ctypes.c_int),
         "vd_kernel_launches": ([], ctypes.c_int64),
         "vd_trim_memory": ([], ctypes.c_int),
+        "vd_path_counts": ([vp, i64p], ctypes.c_int),
         "vd_edges_from_simplices_noalloc": ([ctypes.c_int, vp, i64, i64, vp, i64, i64p, vp], ctypes.c_int),
     }
     for name, (args, res) in sig.items():

@@ -2799,6 +2799,7 @@ __global__ void __launch_bounds__(32) k_finish(DevTree T) {
   flush_tally(ctr, tl, ntests, walk);
   if (lane == 0 && nins > 0) {
     atomicAdd(&ctr->ninserted, nins);
+    atomicAdd(&ctr->nfinished, nins);
     atomicAdd(&ctr->winners, nins);
     atomicAdd(&ctr->created, created);
     atomicAdd(&ctr->killed, killed);

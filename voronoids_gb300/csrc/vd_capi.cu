@@ -189,11 +189,12 @@ struct vd_tree {
     uint64_t seed;
     float ratio;
     long long launches;
-    int64_t call;          // the call that first asked for it
+    int64_t call;          // the call that first asked for it, then the one that captured it
     cudaGraphExec_t exec;  // null: asked for, not captured
   };
   std::vector<ChunkGraph> graphs;
   bool use_graphs = true;
+  int64_t captured = 0, replayed = 0;  // rounds (vd_path_counts)
   bool has_geometry = false;  // a super simplex exists (vd_tree_create leaves none)
   // sets (one unless built by vd_batch_*): first input point of each set
   int nsets = 1;
@@ -816,6 +817,8 @@ vd_tree::ChunkGraph* chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, con
   }
   hit->launches = launches;
   hit->exec = exec;
+  hit->call = t->calls;
+  t->captured += chunk;
   return hit;
 }
 
@@ -838,6 +841,7 @@ bool launch_chunk_graph(vd_tree* t, const vd::Launch& L, int chunk, const vd::Fe
     return false;
   }
   vd::note_launches(g->launches);
+  if (g->call != t->calls) t->replayed += chunk;
   return true;
 }
 
@@ -1581,6 +1585,16 @@ int vd_get_stats(vd_tree* t, vd_stats* s) {
   for (int p = 3; p < vd::kPassesMax; ++p) s->won_pass[2] += (int64_t)h.won[p];
   s->spilled = (int64_t)h.spilled;
   s->max_search_levels = h.max_levels;
+  return VD_OK;
+}
+
+int vd_path_counts(vd_tree* t, int64_t* out) {
+  if (ready(t) || !out) return VD_ERR_ARG;
+  int rc = sync_counters(t);
+  if (rc) return rc;
+  out[0] = t->hctr->nfinished;
+  out[1] = t->captured;
+  out[2] = t->replayed;
   return VD_OK;
 }
 

@@ -111,6 +111,7 @@ struct Counters {
   int bar_abort, coop_go;
   int single;                       // outcome of the last one-point insertion (k_insert_one)
   int nleft;                        // points that k_finish left for the rounds
+  int nfinished;                    // points that k_finish inserted
 };
 
 // Sum of a striped statistics counter (host or device).

@@ -373,6 +373,12 @@ class DelaunayTree:
                               ctypes.byref(n)), "trace")
         return out
 
+    def path_counts(self):
+        """Paths that this tree's work took: see vd_path_counts."""
+        out = np.zeros(3, dtype=np.int64)
+        _check(_native.load().vd_path_counts(self._h, out.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))), "path_counts")
+        return dict(zip(("finished_points", "captured_rounds", "replayed_rounds"), out.tolist()))
+
     def stats(self):
         s = _native.VdStats()
         _check(_native.load().vd_get_stats(self._h, ctypes.byref(s)), "stats")
