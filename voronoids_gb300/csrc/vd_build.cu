@@ -2810,7 +2810,10 @@ __global__ void __launch_bounds__(32) k_finish(DevTree T) {
 }
 
 // Before k_finish, one block: active points that equal one another are left for
-// the rounds, which insert the one of the best priority.  At most kFinishMax points.
+// the rounds, which insert the one of the best priority.  The votes that the
+// points have cast for the next round are taken back: slots are used again, and
+// the vote of a point that is in by then would keep one that is left out of it
+// (k_refit votes for those).  At most kFinishMax points.
 constexpr int kTwinSlots = 2 * kFinishMax;
 __global__ void __launch_bounds__(1024) k_twins(DevTree T) {
   __shared__ int tab[kTwinSlots];
@@ -2839,11 +2842,14 @@ __global__ void __launch_bounds__(1024) k_twins(DevTree T) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int4 e = T.act[par][i];
+    if (!bad_simp(T, e.y)) T.vote[e.y] = ~0ull;
     if (twin[i]) {
-      T.act[par ^ 1][atomicAdd(&ctr->nleft, 1)] = T.act[par][i];
+      T.act[par ^ 1][atomicAdd(&ctr->nleft, 1)] = e;
       T.act[par][i].x = -1;
     }
+  }
 }
 
 // After k_finish, one block: the points it left become the active list of the next
