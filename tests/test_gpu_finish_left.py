@@ -1,4 +1,4 @@
-"""GPU: what k_finish leaves is taken by the next round.
+"""GPU: what k_finish leaves is taken by the next round, and equal points of different sets do not leave one another.
 
 The round before k_finish has each simplex vote for the best of the points in it; votes for points that are in by
 now must not keep a point that is left out of the next round.
@@ -34,4 +34,24 @@ def test_the_next_round_takes_what_is_left(vd, dim):
         assert t.stats()["rounds"] - before == 3
         assert t.path_counts()["finished_points"] > 0 and len(t.duplicates()) == len(centres)
         assert t.check_delaunay()
+    t.close()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_equal_points_of_different_sets(vd, oracle, dim):
+    rng = np.random.default_rng(42)
+    p = rng.random((40, dim))
+    q = np.concatenate([p, p[:9]])[rng.permutation(49)]  # and equal points within a set
+    sets = [p, q, p, q, p, p[::-1].copy(), q, p]
+    t = vd.DelaunayTree.create(dim)
+    off = np.cumsum([0] + [len(s) for s in sets])
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore", RuntimeWarning)
+        uv, eoff = t.batch(np.concatenate(sets), off, seed=3)
+    assert t.path_counts()["finished_points"] >= 100  # of 200 in the sets without equal points
+    for k, s in enumerate(sets):
+        if len(s) == 40:
+            assert np.array_equal(uv[eoff[k]:eoff[k + 1]].astype(np.int64), oracle.Triangulation(s, seed=3).edges())
+    assert len(t.duplicates()) == 3 * 9
+    assert t.check_delaunay()
     t.close()

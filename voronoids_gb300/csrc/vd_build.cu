@@ -2809,7 +2809,7 @@ __global__ void __launch_bounds__(32) k_finish(DevTree T) {
   }
 }
 
-// Before k_finish, one block: active points that equal one another are left for
+// Before k_finish, one block: active points of a set that equal one another are left for
 // the rounds, which insert the one of the best priority.  The votes that the
 // points have cast for the next round are taken back: slots are used again, and
 // the vote of a point that is in by then would keep one that is left out of it
@@ -2825,16 +2825,19 @@ __global__ void __launch_bounds__(1024) k_twins(DevTree T) {
   for (int i = threadIdx.x; i < kFinishMax; i += blockDim.x) twin[i] = 0;
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const vdp::VPt q = load_pt(T, T.act[par][i].x);
+    const int vid = T.act[par][i].x, set = set_index(T, vid);
+    const vdp::VPt q = load_pt(T, vid);
     // -0 and 0 are one value
     const unsigned long long m = (unsigned long long)__double_as_longlong(q.x + 0.0) * 0x9E3779B97F4A7C15ull ^
                                  (unsigned long long)__double_as_longlong(q.y + 0.0) * 0xC2B2AE3D27D4EB4Full ^
-                                 (unsigned long long)__double_as_longlong(q.z + 0.0) * 0x165667B19E3779F9ull;
+                                 (unsigned long long)__double_as_longlong(q.z + 0.0) * 0x165667B19E3779F9ull ^
+                                 (unsigned long long)set * 0xD6E8FEB86659FD93ull;
     unsigned h = (unsigned)((m ^ (m >> 29)) * 0x9E3779B97F4A7C15ull >> 40) & (kTwinSlots - 1);
     for (int probe = 0; probe < kTwinSlots; ++probe, h = (h + 1) & (kTwinSlots - 1)) {
       const int j = atomicCAS(&tab[h], -1, i);
       if (j < 0) break;
-      if (same_point_bits(load_pt(T, T.act[par][j].x), q)) {
+      const int other = T.act[par][j].x;
+      if (set_index(T, other) == set && same_point_bits(load_pt(T, other), q)) {
         twin[i] = 1;
         twin[j] = 1;
         break;
