@@ -273,8 +273,8 @@ int vd_set_trace(vd_tree* t, int on);
 int64_t vd_kernel_launches(void);
 /* Paths that a tree's work took, 3 entries: points of the current triangulation
  * that were inserted under locks at the end of a call instead of in rounds;
- * rounds captured as CUDA graphs since the tree was made; rounds replayed from
- * graphs that an earlier call captured. */
+ * rounds captured as CUDA graphs since the tree was made; rounds of the last
+ * insertion call that were replayed from graphs an earlier call captured. */
 int vd_path_counts(vd_tree* t, int64_t* out);
 int vd_trace(vd_tree* t, int64_t* rows, int64_t cap, int64_t* n);
 

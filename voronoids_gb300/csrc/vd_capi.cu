@@ -194,7 +194,7 @@ struct vd_tree {
   };
   std::vector<ChunkGraph> graphs;
   bool use_graphs = true;
-  int64_t captured = 0, replayed = 0;  // rounds (vd_path_counts)
+  int64_t captured = 0, replayed = 0;  // rounds: all, of the last insertion call (vd_path_counts)
   bool has_geometry = false;  // a super simplex exists (vd_tree_create leaves none)
   // sets (one unless built by vd_batch_*): first input point of each set
   int nsets = 1;
@@ -1067,6 +1067,7 @@ int insert_device(vd_tree* t, const double* d_xyz, int64_t n, uint64_t seed) {
   if (t->hctr->err) return t->hctr->err;
   t->nverts += n;
   t->calls++;
+  t->replayed = 0;
   if (first_block) {
     const int64_t cap = std::min<int64_t>(fb_max, vd::seed_max_points(t->dim));
     int64_t pts = 0;
