@@ -1840,13 +1840,17 @@ int vd_autotune_batch(vd_tree* t, const double* d_pts, const int64_t* offsets, i
     t->tuning.adjacent = c.adjacent;
     t->ratio = c.ratio;
   };
+  // A tuned batch runs again and again on one tree, from captured rounds: the
+  // first build of a configuration asks for its chunks, the second captures them
+  // (0.3 ms a chunk of 8 rounds), and the third, which replays them, is timed.
   auto time_cfg = [&](const Cfg& c) -> double {
     apply(c);
-    double best = 1e30;
-    for (int rep = 0; rep < 2 && !rc; ++rep) {
+    drop_graphs(t);  // another configuration's
+    float ms = 0.f;
+    for (int rep = 0; rep < 3 && !rc; ++rep) {
       cudaEventRecord(e0, t->stream);
       int r = batch_reset_device(t, d_sample, soff.data(), ns);
-      if (!r) r = insert_device(t, d_sample, npts, 0x5eedULL);  // one seed: the second run replays graphs
+      if (!r) r = insert_device(t, d_sample, npts, 0x5eedULL);
       if (r == VD_ERR_DUPLICATE) r = VD_OK;
       if (!r) r = batch_edges(t, d_uv, cap, eoff.data(), nullptr);
       cudaEventRecord(e1, t->stream);
@@ -1855,11 +1859,9 @@ int vd_autotune_batch(vd_tree* t, const double* d_pts, const int64_t* offsets, i
         break;
       }
       cudaEventSynchronize(e1);
-      float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
-      best = std::min(best, (double)ms);
     }
-    return best;
+    return rc ? 1e30 : (double)ms;
   };
   Cfg best{t->warps_per_sm, t->blocks_per_sm, t->tuning.passes, t->tuning.thin, t->tuning.adjacent, t->ratio};
   double best_ms = time_cfg(best);
