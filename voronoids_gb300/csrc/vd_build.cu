@@ -1753,7 +1753,13 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
         // the other facets take the remaining cavity slots, then fresh ones
         for (int i = lane; i < ncav; i += 32) W.first[i] = 0x7fffffff;
         __syncwarp();
-        for (int j = lane; j < nfac; j += 32) atomicMin(&W.first[rec_k(__ldg(F + 6 * j + 5))], j);
+        // (plain loads: the words are written again at the end, and in the small-round
+        // kernel by later rounds, which a non-coherent load need not see)
+        for (int j = lane; j < nfac; j += 32) {
+          const int k = rec_k(F[6 * j + 5]);
+          W.id[j] = k;  // read again below by the same lane
+          atomicMin(&W.first[k], j);
+        }
         __syncwarp();
         int nfree = 0;  // cavity slots without an own facet, ranked
         for (int i0 = 0; i0 < ncav; i0 += 32) {
@@ -1769,7 +1775,7 @@ __device__ __forceinline__ void check_body(DevTree T, int pass, int last, unsign
           int id = 0;
           bool sec = false;
           if (j < nfac) {
-            const int k = rec_k(__ldg(F + 6 * j + 5));
+            const int k = W.id[j];
             sec = W.first[k] != j;
             if (!sec) id = P[k];
           }
