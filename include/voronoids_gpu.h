@@ -336,9 +336,11 @@ vd_tree* vd_tree_create(int dim, void* stream, int* status);
  * them as batched builds, so that requests arriving while others run are
  * admitted as slots and budget free up, and batches of different slots
  * overlap on the device.  Admission: the estimated device bytes of the
- * requests in flight (3D 1850 B/point, 2D 700 B/point, slack included)
- * stay within `pool_bytes`; a request larger than the budget finishes with
- * VD_ERR_NOMEM.  `max_batch_points` caps a batch (0 = only the budget).
+ * requests in flight (3D 2400 B/point, 2D 700 B/point, and for each batch what a
+ * call takes however few its points are: 70 MB in 3D, 54 MB in 2D) stay within
+ * `pool_bytes`, or a batch runs alone.  A request of more than
+ * the budget at 1850 (3D) or 700 B/point (2D) finishes with VD_ERR_NOMEM.
+ * `max_batch_points` caps a batch (0 = only the budget).
  * Each result is the triangulation of the request alone. */
 typedef struct vd_server vd_server;
 vd_server* vd_server_new(uint64_t pool_bytes, int slots, int64_t max_batch_points, uint64_t seed, int* status);

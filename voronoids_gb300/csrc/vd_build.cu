@@ -1126,7 +1126,7 @@ __device__ void big_search(const DevTree& T, WarpCtl& ctl, SearchStats* st, int*
       __syncwarp();
   };
   if (rank == 0) {
-    const int o = atomicAdd(&T.ctr->pool_used, kBigInts + 4);
+    const int o = atomicAdd(&T.ctr->pool_used, kBigInts + 4);  // spill_ints()
     ctl.pad = (o + 3) & ~3;  // int4 alignment of cv / cn
   }
   sync();
@@ -3581,6 +3581,8 @@ int launch_small_rounds(const DevTree& T, cudaStream_t stream, int dim, const Tu
   note_launches(1);
   return E_OK;
 }
+
+int spill_ints() { return kBigInts + 4; }
 
 int search_chunk_ints(int dim) {
   return dim == 3 ? region_ints(Cap<3>::MAXC, Cap<3>::MAXF) : region_ints(Cap<2>::MAXC, Cap<2>::MAXF);

@@ -345,6 +345,17 @@ int ensure_simplices(vd_tree* t, int64_t want) {
   return vd::E_OK;
 }
 
+// Least work pool of a call of n points: six spilled searches and a chunk of every
+// warp that can search in one round.
+int64_t pool_floor_ints(int dim, int sms, int64_t n) {
+  const int64_t warps = std::min<int64_t>(n, (int64_t)sms * kMaxWarpsPerSm);
+  return 6 * vd::spill_ints() + warps * vd::search_chunk_ints(dim);
+}
+
+// Slots that a call sets aside beyond its points' own: what the rounds' warps hold
+// in chunks, and some.
+int64_t spare_slots(int sms) { return 4096 + 32LL * sms * kChunkWarpsPerSm; }
+
 int ensure_points(vd_tree* t, int64_t n_new) {
   int64_t want = t->nverts + n_new;
   if (want > 0x7ffffff0LL) return vd::E_ARG;
@@ -380,12 +391,8 @@ int ensure_points(vd_tree* t, int64_t n_new) {
     t->cap_act = c;
     t->T.cap_cand = (int)c;
   }
-  // room for eight spilled searches and a chunk of every warp that can search
-  // in one round, or what a round of n_new points needs
-  const int64_t warps = std::min<int64_t>(n_new, (int64_t)t->sms * kMaxWarpsPerSm);
   const int64_t pool_want = std::min<int64_t>(
-      std::max<int64_t>((t->dim == 3 ? 48 : 24) * std::max<int64_t>(n_new, 1024),
-                        8 * 360448 + 64 + warps * vd::search_chunk_ints(t->dim)),
+      std::max<int64_t>((t->dim == 3 ? 48 : 24) * std::max<int64_t>(n_new, 1024), pool_floor_ints(t->dim, t->sms, n_new)),
       0x7fffffffLL);
   if (pool_want > t->T.cap_pool) {
     dfree(t->T.pool, t->stream);
@@ -1023,7 +1030,7 @@ int insert_device(vd_tree* t, const double* d_xyz, int64_t n, uint64_t seed) {
   int rc = ensure_points(t, n);
   if (rc) return rc;
   const double per = t->dim == 3 ? 7.6 : 2.3;
-  rc = ensure_simplices(t, t->hctr->nsimp + (int64_t)(per * (double)n) + 4096 + 32LL * t->T.cap_wchunk);
+  rc = ensure_simplices(t, t->hctr->nsimp + (int64_t)(per * (double)n) + spare_slots(t->sms));
   if (rc) return rc;
   t->edges_valid = false;
   const vd::Launch L = launch_of(t);
@@ -1264,6 +1271,18 @@ int batch_edges(vd_tree* t, uint2* d_uv, int64_t cap, int64_t* edge_offsets, int
 }
 
 }  // namespace
+
+namespace vd {
+int64_t call_floor_bytes(int dim) {
+  int dev = 0, sms = 1;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    sms = 1;
+  const int64_t slot = (int64_t)(sizeof(Simplex) + (dim == 3 ? sizeof(vdp::Sph) : 0) + 4 * sizeof(unsigned long long) +
+                                 sizeof(int2) + sizeof(int) + 4 * sizeof(int));
+  return 4 * pool_floor_ints(dim, sms, 0x7fffffff) + slot * spare_slots(sms) + 4 * hint_cells(dim, single_hint_levels(dim));
+}
+}  // namespace vd
 
 // ===========================================================================
 extern "C" {

@@ -321,8 +321,13 @@ struct Prof {
   int type[kMax];
   int n;
 };
-// Pool ints a warp of the region search takes at least at a time.
+// Pool ints a warp of the region search takes at least at a time, and those of a
+// search that spills.
 int search_chunk_ints(int dim);
+int spill_ints();
+// Device bytes that a tree takes for an insertion call however few its points are
+// (work pool, fresh-slot chunks), on the current device.
+int64_t call_floor_bytes(int dim);
 // Kernel attributes the rounds need (shared-memory size); once per context of a
 // device before the first round or capture.
 int prepare_round_kernels();

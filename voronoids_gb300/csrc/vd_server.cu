@@ -25,21 +25,29 @@
 #include <vector>
 
 #include "../../include/voronoids_gpu.h"
+#include "vd_common.cuh"
 
 namespace {
 
-// Estimated device bytes of a request, with slack (3D 1.4x, 2D 1.5x): simplex
-// slots (3D 7.6 per point of 108 B, 2D 2.3 of 92 B: record, stored sphere in
-// 3D, claims, marks, star links) and per-point records, work lists and edge scratch (about 520 B in 3D, 250 B
-// in 2D).
+// Device bytes of a request, by which the budget admits or refuses it on its own.
 int64_t estimate_bytes(int dim, int64_t n) { return (dim == 3 ? 1850 : 700) * std::max<int64_t>(n, 1) + 4096; }
+
+// Device bytes of a request as reserved while it runs.  Simplex slots (3D 7.6 per
+// point of 108 B and, where they do not last, half as many again; 2D 2.3 of 92 B:
+// record, stored sphere in 3D, claims, marks, star links), edge scratch (72 B a
+// simplex in 3D, 36 in 2D), points and work lists (390 B in 3D, 270 in 2D).  Trees
+// of 0.3 to 2 million points hold 2,100 to 2,400 B a point in 3D, 570 in 2D.  A
+// batch also counts what a call takes however few its points are
+// (vd::call_floor_bytes).
+int64_t reserve_bytes(int dim, int64_t n) { return (dim == 3 ? 2400 : 700) * std::max<int64_t>(n, 1) + 4096; }
 
 struct Request {
   int64_t id;
   int dim;
   std::vector<double> pts;
   int64_t n;
-  int64_t bytes;
+  int64_t bytes;    // estimate_bytes
+  int64_t reserve;  // reserve_bytes
   int status = VD_OK;
   std::vector<uint32_t> uv;  // 2 per edge
 };
@@ -132,6 +140,7 @@ void run_batch(vd_server* s, Slot& sl, int dim, std::vector<std::unique_ptr<Requ
 void worker(vd_server* s) {
   cudaSetDevice(s->device);
   Slot sl;
+  const uint64_t floor[2] = {(uint64_t)vd::call_floor_bytes(2), (uint64_t)vd::call_floor_bytes(3)};
   if (cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) != cudaSuccess) sl.stream = nullptr;
   while (true) {
     std::vector<std::unique_ptr<Request>> batch;
@@ -158,18 +167,23 @@ void worker(vd_server* s) {
             s->cv_done.notify_all();
             continue;
           }
-          if (s->reserved + head <= s->budget) {
+          // a batch alone may take the whole budget
+          const bool alone = s->reserved == 0;
+          const uint64_t used = alone ? 0 : s->reserved + floor[q];
+          if (alone || used + (uint64_t)Q.front()->reserve <= s->budget) {
             int64_t pts = 0;
             while (!Q.empty()) {
               Request* r = Q.front().get();
-              const bool room = s->reserved + bytes + (uint64_t)r->bytes <= s->budget;
-              const bool fits = batch.empty() || s->max_batch_points <= 0 || pts + r->n <= s->max_batch_points;
-              if (!room || !fits) break;
+              const bool first = batch.empty();
+              const bool room = used + bytes + (uint64_t)r->reserve <= s->budget;
+              const bool fits = s->max_batch_points <= 0 || pts + r->n <= s->max_batch_points;
+              if (!first && (!room || !fits)) break;
               pts += r->n;
-              bytes += (uint64_t)r->bytes;
+              bytes += (uint64_t)r->reserve;
               batch.push_back(std::move(Q.front()));
               Q.pop_front();
             }
+            bytes = std::min(bytes + floor[q], s->budget - s->reserved);
             dim = q + 2;
             s->reserved += bytes;
             s->peak_reserved = std::max(s->peak_reserved, s->reserved);
@@ -235,6 +249,7 @@ int vd_server_submit(vd_server* s, int dim, const double* pts, int64_t n, int64_
   r->dim = dim;
   r->n = n;
   r->bytes = estimate_bytes(dim, n);
+  r->reserve = reserve_bytes(dim, n);
   r->pts.assign(pts, pts + n * dim);
   {
     std::lock_guard<std::mutex> lk(s->mu);
