@@ -32,9 +32,8 @@
 //               (`insert_points_parallel`, :213-334).  In the default adjacent
 //               mode a decide half and a commit half are separate kernels, and
 //               the stars of winners that share a facet are stitched at the
-//               start of k_relocate.  A round equals some sequential insertion
-//               order.  k_reclaim (and k_relocate for the last pass) also makes
-//               the stored spheres of the stars just written.
+//               start of k_relocate, which also makes the stored spheres of
+//               the stars.  A round equals some sequential insertion order.
 //   k_relocate  one thread per uninserted point: points whose simplex was
 //               removed walk inside the new star (faces through the new vertex
 //               only) to the simplex that contains them; every point then votes

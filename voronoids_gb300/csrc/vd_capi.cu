@@ -1059,7 +1059,7 @@ int insert_device(vd_tree* t, const double* d_xyz, int64_t n, uint64_t seed) {
   cudaMemsetAsync(t->d_counts, 0, sizeof(int) * 2 * vd::kMaxLevels, t->stream);
   vd::launch_levels(t->T, L, n, base, seed, thr.data(), (int)thr.size(), first, t->growth, t->d_counts);
   // a fresh single-set call starts with its first levels in one block
-    // (about 2 us a point in 3D, 1.6 in 2D; up to 150 / 250 / 370 / 525 points a
+  // (about 2 us a point in 3D, 1.6 in 2D; up to 150 / 250 / 370 / 525 points a
   // 1,000-point build takes 3.19 / 2.89 / 2.80 / 2.90 ms in 3D and 1.66 / 1.60 /
   // 1.64 / 1.73 in 2D, 262,144 points 19.2 / 18.8 / 18.4 / 18.6 in 3D, 1M points
   // 15.9 / 15.2 / 15.4 / 15.3 in 2D)
