@@ -1,4 +1,4 @@
-"""GPU: trees made after the device's context was reset.
+"""GPU: trees made after the device's context was reset, and by threads that make their first CUDA call with one.
 
 In a process of its own: builds through every kind of call, a reset of the context
 with no tree alive (the caller holds nothing of the library then), and the same
@@ -57,3 +57,25 @@ print("same edges")
 def test_builds_after_a_context_reset():
     r = subprocess.run([sys.executable, "-c", CHILD], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same edges" in r.stdout, r.stdout + r.stderr
+
+
+def test_first_call_of_a_thread(vd, oracle):
+    import threading
+
+    from voronoids_gb300 import workloads as W
+    p = W.uniform_points(4000, 3, 71)
+    want = oracle.Triangulation(p, seed=1).edges()
+    good = []
+
+    def build():
+        t = vd.delaunay(p, seed=1)
+        good.append((t.edges() == want).all())
+        t.close()
+
+    for _ in range(3):  # blocks that one thread gives back are another's
+        threads = [threading.Thread(target=build) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert good == [True] * 12

@@ -26,18 +26,20 @@ STAND_IN = r"""
 namespace {
 unsigned long long last_id = 2, ctx_of[2] = {1, 2};  // of devices 0 and 1
 int dev = 0, faults = 0, pinned_made = 0;
+bool bound = true;  // the thread has a current context
 std::map<void*, unsigned long long> pools, blocks, pinned;  // handle or block -> its context
 bool alive(const std::map<void*, unsigned long long>& m, void* p) {
   auto i = m.find(p);
   return i != m.end() && (i->second == ctx_of[0] || i->second == ctx_of[1]);
 }
-CUresult ctx_get(CUcontext* c) { *c = (CUcontext)(size_t)ctx_of[dev]; return CUDA_SUCCESS; }
+CUresult ctx_get(CUcontext* c) { *c = bound ? (CUcontext)(size_t)ctx_of[dev] : nullptr; return CUDA_SUCCESS; }
 CUresult ctx_id(CUcontext c, unsigned long long* id) { *id = (size_t)c; return CUDA_SUCCESS; }
 }  // namespace
 namespace vd { void note_launches(long long) {} }
 
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = dev; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { dev = d; bound = true; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 1; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
@@ -74,6 +76,7 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigne
 }
 
 void on_device(int d) { dev = d; }
+void unbind(void) { bound = false; }
 void reset(void) { ctx_of[dev] = ++last_id; }
 int fault_count(void) { return faults; }
 int made_count(void) { return pinned_made; }
@@ -160,3 +163,10 @@ def test_a_trim_after_a_reset_touches_nothing_dead(mem):
     assert mem.usable(mem.take()) and mem.made_count() == 2  # the kept block was given back
     mem.reset()
     assert mem.trim() == 0 and mem.array() and mem.fault_count() == 0
+
+
+def test_a_thread_without_a_context_gets_its_devices(mem):
+    p = mem.take()
+    mem.give(p, mem.taken_owner())
+    mem.unbind()  # as in a new thread
+    assert mem.take() == p and mem.usable(p) and mem.array() and mem.fault_count() == 0

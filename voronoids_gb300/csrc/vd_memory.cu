@@ -52,8 +52,9 @@ ContextMemory* entry_of(unsigned long long id) {  // g_mu held
 // (then allocations are plain).  g_mu held.
 ContextMemory* current_entry() {
   unsigned long long id = context_id();
-  if (id == 0) {
-    cudaFree(nullptr);  // a thread's first call: binds its device's context
+  int dev = 0, has = 0;
+  if (id == 0 && cudaGetDevice(&dev) == cudaSuccess) {
+    cudaSetDevice(dev);  // a thread's first call: binds its device's context (other threads may be capturing)
     id = context_id();
   }
   if (id == 0) return nullptr;
@@ -61,7 +62,6 @@ ContextMemory* current_entry() {
   ContextMemory& e = g_mem[g_next];
   g_next = (g_next + 1) % kContexts;
   e = ContextMemory{};
-  int dev = 0, has = 0;
   cudaMemPoolProps props = {};
   unsigned long long keep = kKeepBytes;
   if (cudaGetDevice(&dev) == cudaSuccess) {
